@@ -60,18 +60,27 @@ __global__ void __launch_bounds__(512) ep_push_rows_kernel(const __nv_bfloat16* 
 
 // Router and push in one launch: every CTA (one per destination rank) routes all B rows itself — the routing is a deterministic
 // function of the logits, so the G copies agree — and sends rows, ids and weights to its rank.  CTA 0 also stores ids / w for
-// the caller.  Dynamic shared memory: (warps·E + 2·B·K) words.
+// the caller.  A row goes to a group of ep_route_warps(B) of the 16 warps.  Dynamic
+// shared memory: (16 / warps a row · E + 2·B·K) words.
+__host__ __device__ inline int ep_route_warps(int B) { return B <= 1 ? 16 : B <= 2 ? 8 : B <= 4 ? 4 : 2; }
 __global__ void __launch_bounds__(512) ep_route_push_kernel(const float* __restrict__ logits, int ld, int E, int K, int renorm, int logits_bf16,
                                                             const __nv_bfloat16* __restrict__ x, int ldx, int32_t* __restrict__ ids_out,
                                                             float* __restrict__ w_out, int B, int H, int rec_bytes, EpPeers peers, int rank,
                                                             const uint32_t* __restrict__ step_ctr) {
   extern __shared__ float ep_sm[];
+  __shared__ RouteShare rs[8];
   griddep_wait();                                                          // the previous step's combine has advanced the step counter
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  int32_t* ids_s = reinterpret_cast<int32_t*>(ep_sm + (size_t)nw * E);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = ep_route_warps(B), grp = warp / W, ngrp = 16 / W;
+  float* p = ep_sm + (size_t)grp * E;
+  int32_t* ids_s = reinterpret_cast<int32_t*>(ep_sm + (size_t)ngrp * E);
   float* w_s = reinterpret_cast<float*>(ids_s + B * K);
-  for (int m = warp; m < B; m += nw)
-    route_softmax_row(logits + (size_t)m * ld, E, K, renorm, logits_bf16, ep_sm + (size_t)warp * E, lane, ids_s + m * K, w_s + m * K);
+  const RouteArgs ra{1, E, K, renorm, logits_bf16, nullptr, 1.f};
+  const RouteGroup rg{warp - grp * W, W, 1 + grp};
+  for (int m = grp; m < B; m += ngrp) {
+    int id; float wv;
+    route_row<false>(ra, logits + (size_t)m * ld, p, rs[grp], rg, lane, id, wv);
+    if (rg.warp == 0 && lane < K) { ids_s[m * K + lane] = id; w_s[m * K + lane] = wv; }
+  }
   __syncthreads();
   const int pi = blockIdx.x;
   if (pi == 0)
@@ -250,8 +259,8 @@ int hb_ep_route_push(hb_ep* e, const float* logits, int ld, int E, int renorm, i
   hb_ctx* ctx = e->ctx;
   HB_REQUIRE(ctx, logits && x_bf16 && ids_out && w_out && ldx >= e->H && ldx % 8 == 0 && hb_aligned(x_bf16, 16), HB_ERR_INVALID, "ep_route_push: bad arguments");
   HB_REQUIRE(ctx, E >= 1 && ld >= E && e->K <= 16 && e->K <= E, HB_ERR_INVALID, "ep_route_push: E=%d ld=%d K=%d", E, ld, e->K);
-  const size_t smem = ((size_t)16 * E + 2 * (size_t)e->B * e->K) * 4;
-  HB_REQUIRE(ctx, smem <= 48 * 1024, HB_ERR_UNSUPPORTED, "ep_route_push: E=%d too large for the fused router (route with hb_route_softmax_topk, then hb_ep_push_rows)", E);
+  HB_REQUIRE(ctx, ((size_t)16 * E + 2 * (size_t)e->B * e->K) * 4 <= 48 * 1024, HB_ERR_UNSUPPORTED, "ep_route_push: E=%d too large for the fused router (route with hb_route_softmax_topk, then hb_ep_push_rows)", E);
+  const size_t smem = ((size_t)(16 / ep_route_warps(e->B)) * E + 2 * (size_t)e->B * e->K) * 4;
   return hb_launch(ctx, "ep_route_push", true, ep_route_push_kernel, dim3(e->world), dim3(512), smem, reinterpret_cast<cudaStream_t>(stream), logits, ld, E,
                    e->K, renorm, logits_bf16, reinterpret_cast<const __nv_bfloat16*>(x_bf16), ldx, ids_out, w_out, e->B, e->H, e->rec_bytes, e->peers, e->rank,
                    (const uint32_t*)e->step_ctr);

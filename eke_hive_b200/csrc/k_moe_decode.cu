@@ -27,140 +27,169 @@ struct GroupArgs {
   int ld_ids, sh_row0, sh_rows;                          // pitch of ids / w rows; rows [sh_row0, sh_row0 + sh_rows) get the shared pair
   const uint32_t* wait_flags; int wait_n; const uint32_t* wait_step; uint32_t* wait_err;   // expert parallel: the gathered rows' flags
   DecodeWs ws;
-  // optional routing stage (routed form): logits → ids / w by one warp per row before the grouping
-  int route; const float* logits; int ld, renorm, logits_bf16; const float* bias; float sig_scale;
+  // optional routing stage (routed form): logits → ids / w before the grouping
+  RouteArgs rt; const float* logits; int ld;
   int32_t* ids_out; float* w_out;
-  int group_rows;       // rows per group (≤ kGroupRows)
+  uint32_t k_inv;       // ceil(2^32 / K): i / K is the high word of i · k_inv (i, K ≤ HB_MAX_PAIRS; not for K = 1)
+  int group_shift;      // log2 of the rows per group (≤ kGroupRows)
 };
-
-// Exclusive scan of two int arrays of length n in shared memory, by the whole block (blockDim.x == kGroupThreads).
-__device__ void block_scan2(int* a, int* b, int n, int* tot_a, int* tot_b, int* warp_tmp /* [2][32] */) {
-  const int per = (n + kGroupThreads - 1) / kGroupThreads;
-  const int i0 = threadIdx.x * per, i1 = min(n, i0 + per);
-  int sa = 0, sb = 0;
-  for (int i = i0; i < i1; ++i) { sa += a[i]; sb += b[i]; }
-  int xa = sa, xb = sb;                                  // inclusive warp scan of the per-thread sums
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int ta = __shfl_up_sync(0xffffffffu, xa, o), tb = __shfl_up_sync(0xffffffffu, xb, o);
-    if (lane >= o) { xa += ta; xb += tb; }
-  }
-  if (lane == 31) { warp_tmp[warp] = xa; warp_tmp[32 + warp] = xb; }
-  __syncthreads();
-  if (warp == 0) {
-    int va = warp_tmp[lane], vb = warp_tmp[32 + lane];
-    const int ia = va, ib = vb;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int ta = __shfl_up_sync(0xffffffffu, va, o), tb = __shfl_up_sync(0xffffffffu, vb, o);
-      if (lane >= o) { va += ta; vb += tb; }
-    }
-    warp_tmp[lane] = va - ia; warp_tmp[32 + lane] = vb - ib;          // exclusive warp offsets
-    if (lane == 31) { *tot_a = va; *tot_b = vb; }
-  }
-  __syncthreads();
-  int ba = warp_tmp[warp] + xa - sa, bb = warp_tmp[32 + warp] + xb - sb;
-  for (int i = i0; i < i1; ++i) { const int ca = a[i], cb = b[i]; a[i] = ba; b[i] = bb; ba += ca; bb += cb; }
-  __syncthreads();
-}
 
 constexpr int kTcGuMinPairs = 40;                   // unpinned contexts: pairs per call from which gate/up runs on the tensor-memory kernel
 
-__global__ void __launch_bounds__(kGroupThreads) moe_group_kernel(GroupArgs a) {
+// Sorts the pairs by expert: counts the pairs of every expert, scans the counts, places the pairs.  It sits alone on the critical path in
+// front of the two weight passes, so what bounds it is its chain of loads, instructions and block barriers: the counters are cleared
+// before the wait for the previous kernel, the record table is fetched before the ids are there, a pair's slot inside its expert's run
+// is what the counting atomic returned, and both scans (pairs, groups) run as one on packed 16-bit halves.
+// ROUTE: the rows are routed first, by a cluster of kRouteCtas CTAs (grid = one cluster) that share the rows out — one CTA alone was
+// bound by the instructions of its rows (see router.cuh) — and hand the ids to the first CTA through its shared memory; the others
+// then leave.  Without: one CTA, ids given or list form.  Measured, wait for the previous kernel to end of kernel, against one CTA with a
+// warp a row (512 experts, top-10; last: 160 experts, sigmoid): 1 row 6.0 vs 7.2 µs, 16 rows 6.8 vs 12.9, 45 rows 11 vs 32, 8 rows 5.8 vs 18.
+constexpr int kRouteCtas = 8;
+constexpr int kGroupWarps = kGroupThreads / 32;
+// A cluster costs a barrier across its CTAs (0.7 µs, measured in the kernel): one or two rows stay in one CTA.
+__host__ __device__ constexpr int route_ctas(int M) { return M <= 2 ? 1 : kRouteCtas; }
+__host__ __device__ constexpr int route_wlog(int M) {     // log2 of the warps a row gets: as many as keep every warp of a CTA busy (at most 8 named barriers)
+  const int rows = (M + route_ctas(M) - 1) / route_ctas(M);
+  return rows <= 1 ? 4 : rows <= 2 ? 3 : rows <= 4 ? 2 : 1;
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+
+template <int CTAS>
+__device__ __forceinline__ void group_body(const GroupArgs& a) {
   extern __shared__ __align__(16) uint8_t gsm[];
+  __shared__ uint32_t warp_sum[32];
+  constexpr bool ROUTE = CTAS > 0;
+  const bool routed = ROUTE || a.ids != nullptr;
+  const int MK = a.M * a.K;
+  const int P = routed ? MK + (a.shared_rec ? a.M : 0) : a.n_pairs;
+  const int NK = routed ? a.E + 1 : P;                  // key space: expert id (E = the shared expert) or leader pair index
+  constexpr int nt = kGroupThreads, nw = kGroupWarps;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint8_t** recs = reinterpret_cast<const uint8_t**>(gsm);       // [P], list form only
+  uint32_t* key = reinterpret_cast<uint32_t*>(recs + (routed ? 0 : P));   // [P] expert id → key << 16 | slot inside the key's run, ~0 = skipped
+  uint32_t* cnt = key + P;                                             // [NK] pairs of the key → first position of its run, kNoRec without a record
+  constexpr uint32_t kNoRec = 0x80000000u;
+  for (int k = tid; k < NK; k += nt) cnt[k] = 0u;
+  if (CTAS > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");   // every CTA of the cluster is there before the first writes into another's memory
   griddep_wait();
   griddep_launch();                                     // what follows in the stream may start its prologue (each kernel waits for its own inputs)
   if (a.wait_flags) {                                   // the rows, ids and weights this pass reads are pushed by the other ranks
-    if ((int)threadIdx.x < a.wait_n && !*reinterpret_cast<volatile uint32_t*>(a.wait_err))
-      ep_wait_flag(a.wait_flags + threadIdx.x, *a.wait_step + 1u, a.wait_err, 0x40000u);
+    if (tid < a.wait_n && !*reinterpret_cast<volatile uint32_t*>(a.wait_err))
+      ep_wait_flag(a.wait_flags + tid, *a.wait_step + 1u, a.wait_err, 0x40000u);
     __syncthreads();
   }
-  const bool routed = a.ids != nullptr;
-  const int P = routed ? a.M * a.K + (a.shared_rec ? a.M : 0) : a.n_pairs;
-  const int NK = routed ? a.E + 1 : P;                  // key space: expert id (E = the shared expert) or leader pair index
-  int* key = reinterpret_cast<int*>(gsm);               // [P]
-  int* cnt = key + P;                                   // [NK] → exclusive offsets
-  int* ngr = cnt + NK;                                  // [NK] → exclusive group bases
-  int* fill = ngr + NK;                                 // [NK]
-  int* misc = fill + NK;                                // [64 + 2]
-  const uint8_t** recs = reinterpret_cast<const uint8_t**>(gsm + ((size_t)(P + 3 * NK + 68) * 4 + 7) / 8 * 8);   // [P], list form only
-  if (a.route) {                                        // routed form with routing: recs is unused, the router scratch sits there
-    float* rsm = reinterpret_cast<float*>(recs);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    for (int m = warp; m < a.M; m += nwarps) {
-      if (a.route == 1) route_softmax_row(a.logits + (size_t)m * a.ld, a.E, a.K, a.renorm, a.logits_bf16, rsm + (size_t)warp * a.E, lane,
-                                          a.ids_out + (size_t)m * a.K, a.w_out + (size_t)m * a.K);
-      else route_sigmoid_row(a.logits + (size_t)m * a.ld, a.bias, a.E, a.K, a.sig_scale, rsm + (size_t)warp * 2 * a.E, lane,
-                             a.ids_out + (size_t)m * a.K, a.w_out + (size_t)m * a.K);
+  const int per = (NK + nt - 1) / nt, k0 = tid * per, k1 = min(NK, k0 + per);   // keys of this thread
+  auto row_of = [&](int i) { return a.K == 1 ? i : (int)__umulhi((uint32_t)i, a.k_inv); };   // i / K
+  const uint8_t* const* tab = a.tab + (size_t)a.li * a.E;
+  const uint8_t* rec0 = nullptr;                        // the record of the thread's first key
+  if (ROUTE) {
+    const int cta = CTAS > 1 ? (int)cluster_rank() : 0;
+    if (cta == 0 && k0 < k1) rec0 = k0 == a.E ? a.shared_rec : tab[k0];
+    if (CTAS > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    const int wlog = route_wlog(a.M), grp = warp >> wlog, groups = nw >> wlog;
+    const RouteGroup rg{warp - (grp << wlog), 1 << wlog, 1 + grp};
+    RouteShare* rs = reinterpret_cast<RouteShare*>(gsm + (((size_t)(P + NK) * 4 + 15) & ~(size_t)15));
+    float* p = reinterpret_cast<float*>(rs + groups) + (size_t)grp * a.E;
+    uint32_t rkey = smem_u32(key);                      // the first CTA's list of ids
+    if (CTAS > 1) asm volatile("mapa.shared::cluster.u32 %0, %0, 0;" : "+r"(rkey));
+    for (int m = cta + grp * CTAS; m < a.M; m += groups * CTAS) {
+      int id; float wv;
+      if (a.rt.kind == 1) route_row<false>(a.rt, a.logits + (size_t)m * a.ld, p, rs[grp], rg, lane, id, wv);
+      else route_row<true>(a.rt, a.logits + (size_t)m * a.ld, p, rs[grp], rg, lane, id, wv);
+      if (rg.warp == 0 && lane < a.K) {
+        const int i = m * a.K + lane;
+        if (CTAS > 1) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(rkey + 4u * (uint32_t)i), "r"(id) : "memory");
+        else key[i] = (uint32_t)id;
+        a.ids_out[i] = id; a.w_out[i] = wv; a.ws.pw[i] = wv;
+      }
     }
-    __syncthreads();                                    // ids / w of every row are written (same CTA): the grouping below reads them
-  }
-  for (int k = threadIdx.x; k < NK; k += blockDim.x) { cnt[k] = 0; fill[k] = 0; }
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    int row, kk = -1; float wv;
-    if (routed) {
-      if (i < a.M * a.K) {
-        row = i / a.K;
-        const size_t src = (size_t)row * a.ld_ids + (i - row * a.K);
-        const int e = a.ids[src];
-        wv = a.w[src];
-        if (e >= 0 && e < a.E && a.tab[(size_t)a.li * a.E + e] != nullptr) kk = e;
-      } else { row = i - a.M * a.K; wv = 1.f; kk = row >= a.sh_row0 && row < a.sh_row0 + a.sh_rows ? a.E : -1; }
-    } else {
+    if (CTAS > 1) {
+      asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (cta != 0) return;
+    } else __syncthreads();
+  } else if (routed) {
+    if (k0 < k1) rec0 = k0 == a.E ? a.shared_rec : tab[k0];
+    for (int i = tid; i < MK; i += nt) {
+      const int row = row_of(i);
+      const size_t src = (size_t)row * a.ld_ids + (i - row * a.K);
+      key[i] = (uint32_t)a.ids[src]; a.ws.pw[i] = a.w[src];
+    }
+    __syncthreads();
+  } else {
+    for (int i = tid; i < P; i += nt) {
       const hb_moe_pair p = a.pairs[i];
-      row = p.row; wv = p.w; recs[i] = p.rec;
-      kk = p.rec ? i : -1;                              // replaced by the leader index below
-    }
-    key[i] = kk; a.ws.prow[i] = row; a.ws.pw[i] = wv;
-  }
-  __syncthreads();
-  if (!routed) {
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-      const uint8_t* r = recs[i];
-      if (!r) continue;
-      int l = i;
-      for (int j = 0; j < i; ++j) if (recs[j] == r) { l = j; break; }
-      key[i] = l;
+      recs[i] = p.rec;
+      a.ws.prow[i] = p.row; a.ws.pw[i] = p.w;
     }
     __syncthreads();
   }
-  for (int i = threadIdx.x; i < P; i += blockDim.x) if (key[i] >= 0) atomicAdd(&cnt[key[i]], 1);
-  __syncthreads();
-  const int GR = a.group_rows;                          // rows per group: 8 for the streaming gate/up kernel, 2 for the tensor-memory one
-  for (int k = threadIdx.x; k < NK; k += blockDim.x) ngr[k] = (cnt[k] + GR - 1) / GR;
-  __syncthreads();
-  // keep the counts: the scan overwrites cnt with offsets, so copy them into fill's slot first (fill is re-zeroed after)
-  for (int k = threadIdx.x; k < NK; k += blockDim.x) fill[k] = cnt[k];
-  __syncthreads();
-  block_scan2(cnt, ngr, NK, &misc[64], &misc[65], misc);
-  // groups of every key that has pairs
-  for (int k = threadIdx.x; k < NK; k += blockDim.x) {
-    const int c = fill[k];
-    if (c == 0) continue;
-    const uint8_t* rec = routed ? (k == a.E ? a.shared_rec : a.tab[(size_t)a.li * a.E + k]) : recs[k];
-    for (int j = 0; j * GR < c; ++j)
-      if (HB_BOUND(a.wait_err, ngr[k] + j >= 0 && ngr[k] + j < P, 0x101u, ngr[k] + j))
-        a.ws.groups[ngr[k] + j] = Group{rec, cnt[k] + j * GR, min(GR, c - j * GR)};
+  for (int i = tid; i < P; i += nt) {
+    uint32_t kk = ~0u;
+    if (!routed) {
+      const uint8_t* r = recs[i];
+      if (r) { kk = (uint32_t)i; for (int j = 0; j < i; ++j) if (recs[j] == r) { kk = (uint32_t)j; break; } }   // the first pair with this record stands for it
+    } else if (i < MK) kk = key[i] < (uint32_t)a.E ? key[i] : ~0u;
+    else {                                              // one pair of weight 1 per row for the shared expert
+      const int row = i - MK;
+      kk = row >= a.sh_row0 && row < a.sh_row0 + a.sh_rows ? (uint32_t)a.E : ~0u;
+      a.ws.pw[i] = 1.f;
+    }
+    key[i] = kk == ~0u ? ~0u : kk << 16 | atomicAdd(&cnt[kk], 1u);
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < NK; k += blockDim.x) fill[k] = 0;
+  // exclusive scan over the keys of (pairs, groups), 16 bits each (at most HB_MAX_PAIRS = 4096 of either)
+  auto rec_of = [&](int k) { return !routed ? recs[k] : k == k0 ? rec0 : k == a.E ? a.shared_rec : tab[k]; };
+  const int gs = a.group_shift, gm = (1 << gs) - 1;     // rows per group: 8 for the streaming gate/up kernel, 2 for the tensor-memory one
+  uint32_t mine = 0u;
+  for (int k = k0; k < k1; ++k) {
+    uint32_t c = cnt[k];
+    if (c && !rec_of(k)) { c = 0u; cnt[k] = kNoRec; }   // an expert without a record: its pairs are skipped
+    mine += c | ((c + gm) >> gs) << 16;
+  }
+  uint32_t incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+  if (lane == 31) warp_sum[warp] = incl;
   __syncthreads();
-  // slot inside the expert's run: any order gives the same results (columns of a tile are independent)
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    const int kk = key[i];
+  const uint32_t wsum = lane < nw ? warp_sum[lane] : 0u;
+  uint32_t run = incl - mine + __reduce_add_sync(0xffffffffu, lane < warp ? wsum : 0u);
+  for (int k = k0; k < k1; ++k) {                       // groups of every key that has pairs
+    const int c = (int)cnt[k], pos = (int)(run & 0xffffu), g0 = (int)(run >> 16);
+    if (c <= 0) continue;
+    cnt[k] = (uint32_t)pos;
+    const uint8_t* rec = rec_of(k);
+    int j = 0;
+#pragma unroll 1
+    for (int r0 = 0; r0 < c; r0 += gm + 1, ++j)
+      if (HB_BOUND(a.wait_err, g0 + j >= 0 && g0 + j < P, 0x101u, g0 + j)) a.ws.groups[g0 + j] = Group{rec, pos + r0, min(gm + 1, c - r0)};
+    run += (uint32_t)c | (uint32_t)j << 16;
+  }
+  if (warp == 0) {
+    const uint32_t total = __reduce_add_sync(0xffffffffu, wsum);
+    if (lane == 0) *reinterpret_cast<int4*>(a.ws.hdr) = make_int4((int)(total >> 16), (int)(total & 0xffffu), 0, 0);
+  }
+  __syncthreads();
+  // the slot inside an expert's run: any order gives the same results (columns of a tile are independent)
+  for (int i = tid; i < P; i += nt) {
+    const uint32_t kr = key[i], base = kr == ~0u ? kNoRec : cnt[kr >> 16];
     int pos = -1;
-    if (kk >= 0) { pos = cnt[kk] + atomicAdd(&fill[kk], 1); if (HB_BOUND(a.wait_err, pos >= 0 && pos < P, 0x102u, pos)) a.ws.s_row[pos] = a.ws.prow[i]; }
+    if (base != kNoRec) {
+      pos = (int)(base + (kr & 0xffffu));
+      const int row = !routed ? a.ws.prow[i] : i < MK ? row_of(i) : i - MK;
+      if (HB_BOUND(a.wait_err, pos >= 0 && pos < P, 0x102u, pos)) a.ws.s_row[pos] = row;
+    }
     a.ws.pos_of[i] = pos;
+    a.ws.done[i] = 0;
   }
-  for (int i = threadIdx.x; i < P; i += blockDim.x) a.ws.done[i] = 0;
-  if (threadIdx.x == 0) { a.ws.hdr[0] = misc[65]; a.ws.hdr[1] = misc[64]; a.ws.hdr[2] = 0; a.ws.hdr[3] = 0; }
 }
+__global__ void __launch_bounds__(kGroupThreads) moe_group_kernel(const GroupArgs a) { group_body<0>(a); }
+__global__ void __launch_bounds__(kGroupThreads) moe_route_group1_kernel(const GroupArgs a) { group_body<1>(a); }
+__global__ void __cluster_dims__(kRouteCtas, 1, 1) __launch_bounds__(kGroupThreads) moe_route_group_kernel(const GroupArgs a) { group_body<kRouteCtas>(a); }
 
-static size_t group_smem(bool routed, int P, int E, int route = 0) {
-  const int NK = routed ? E + 1 : P;
-  size_t b = (size_t)P * 4 + (size_t)NK * 12 + 68 * 4;
-  b = (b + 7) / 8 * 8;
-  if (route) return b + (size_t)(kGroupThreads / 32) * E * 4 * (route == 2 ? 2 : 1);
-  return b + (routed ? 0 : (size_t)P * 8);
+static size_t group_smem(bool routed, int P, int E, bool route, int M) {
+  size_t b = (size_t)P * 4 + (routed ? ((size_t)E + 1) * 4 : (size_t)P * 12);
+  if (route) b = ((b + 15) & ~(size_t)15) + (kGroupWarps >> route_wlog(M)) * (sizeof(RouteShare) + (size_t)E * 4);
+  return b;
 }
 
 // ================================================================================================ streaming kernels
@@ -477,7 +506,7 @@ using namespace hb;
 namespace {
 
 constexpr int kWkList[] = {1, 2, 3, 4, 6, 8, 12, 16};
-constexpr size_t kRouteSmemMax = 160 * 1024;       // shared memory the route + group kernel may ask for
+constexpr size_t kGroupSmemMax = 64 * 1024;        // shared memory the grouping kernels ask for at most: 16 bytes a pair, HB_MAX_PAIRS of them, or the router's arrays
 constexpr int wm_for(int wk) { return wk >= 8 ? 1 : (wk >= 4 ? 2 : (wk == 3 ? 2 : (wk == 2 ? 4 : 8))); }
 
 using StreamFn = void (*)(StreamArgs);
@@ -559,8 +588,8 @@ int hbk_moe_decode_setup(hb_ctx* ctx) {
     if (!rf) rf = hbk_moe_dtc_setup(ctx);
     if (rf) return rf;
   }
-  HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(moe_group_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kRouteSmemMax));
+  for (const void* fn : {reinterpret_cast<const void*>(moe_group_kernel), reinterpret_cast<const void*>(moe_route_group1_kernel), reinterpret_cast<const void*>(moe_route_group_kernel)})
+    HB_CUDA(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGroupSmemMax));
   return HB_OK;
 }
 
@@ -593,23 +622,16 @@ int hbk_moe_decode_run(hb_ctx* ctx, const hbk_pair_src& src, const void* x, int 
     const bool auto_tc = pairs_eff >= kTcGuMinPairs && (ranks == 1 || src.M <= 64);
     tc_gu = (ctx->flags & (HB_FLAG_DECODE_TC_GU | HB_FLAG_DECODE_TC)) || auto_tc;
   }
-  ga.group_rows = tc_gu ? 2 : kGroupRows;
+  ga.group_shift = tc_gu ? 1 : 3;
   const int x_ld = src.x_ld ? src.x_ld : H;
   if (src.route && ga.ld_ids != src.K) return hb_fail(ctx, HB_ERR_INVALID, "moe_decode: in-kernel routing writes dense ids / w rows");
-  int route = src.route;
-  if (route && group_smem(true, P, src.E, route) > kRouteSmemMax) {
-    // the per-warp router scratch does not fit beside the grouping arrays (large E): route with the stand-alone kernel first
-    int rr = route == 1 ? hbk_route_softmax_topk(ctx, src.logits, src.ld, src.M, src.E, src.K, src.renorm, src.logits_bf16, const_cast<int32_t*>(src.ids),
-                                                 const_cast<float*>(src.w), st, true)
-                        : hbk_route_sigmoid_topk(ctx, src.logits, src.bias, src.M, src.E, src.K, src.sig_scale, const_cast<int32_t*>(src.ids),
-                                                 const_cast<float*>(src.w), st, true);
-    if (rr) return rr;
-    route = 0;
-  }
-  ga.route = route; ga.logits = src.logits; ga.ld = src.ld; ga.renorm = src.renorm; ga.logits_bf16 = src.logits_bf16; ga.bias = src.bias;
-  ga.sig_scale = src.sig_scale; ga.ids_out = const_cast<int32_t*>(src.ids); ga.w_out = const_cast<float*>(src.w);
-  int r = hb_launch(ctx, route ? "moe_route_group" : "moe_group", true, moe_group_kernel, dim3(1), dim3(kGroupThreads), group_smem(routed, P, src.E, route),
-                    st, ga);
+  ga.rt = RouteArgs{src.route, src.E, src.K, src.renorm, src.logits_bf16, src.bias, src.sig_scale};
+  ga.logits = src.logits; ga.ld = src.ld; ga.ids_out = const_cast<int32_t*>(src.ids); ga.w_out = const_cast<float*>(src.w);
+  const size_t gsmem = group_smem(routed, P, src.E, src.route != 0, src.M);
+  ga.k_inv = src.K > 1 ? (uint32_t)(((1ull << 32) + src.K - 1) / src.K) : 0u;
+  const int ctas = src.route ? route_ctas(src.M) : 1;
+  int r = hb_launch(ctx, src.route ? "moe_route_group" : "moe_group", true, !src.route ? moe_group_kernel : ctas == 1 ? moe_route_group1_kernel : moe_route_group_kernel,
+                    dim3(ctas), dim3(kGroupThreads), gsmem, st, ga);
   if (r) return r;
 
   StreamArgs sa{};

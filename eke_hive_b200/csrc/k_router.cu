@@ -6,25 +6,20 @@
 
 namespace hb {
 
-// One warp per row (see router.cuh)
-__global__ void router_softmax_kernel(const float* __restrict__ logits, int ld, int M, int E, int k, int renorm, int logits_bf16,
-                                      int32_t* __restrict__ ids, float* __restrict__ w) {
-  extern __shared__ float sm_p[];
-  griddep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (m >= M) return;
-  route_softmax_row(logits + (size_t)m * ld, E, k, renorm, logits_bf16, sm_p + (size_t)warp * E, lane, ids + (size_t)m * k, w + (size_t)m * k);
-}
+constexpr int kRouterWarps = 4;
 
-__global__ void router_sigmoid_kernel(const float* __restrict__ logits, const float* __restrict__ bias, int M, int E, int k, float scale,
-                                      int32_t* __restrict__ ids, float* __restrict__ w) {
+// One warp per row (see router.cuh): many rows, so throughput counts and not one row's latency.  Dynamic shared memory: E floats a warp.
+template <bool SIG>
+__global__ void router_kernel(const RouteArgs a, const float* __restrict__ logits, int ld, int M, int32_t* __restrict__ ids, float* __restrict__ w) {
   extern __shared__ float sm_p[];
+  __shared__ RouteShare rs[kRouterWarps];
   griddep_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = blockIdx.x * (blockDim.x >> 5) + warp;
+  const int m = blockIdx.x * kRouterWarps + warp;
   if (m >= M) return;
-  route_sigmoid_row(logits + (size_t)m * E, bias, E, k, scale, sm_p + (size_t)warp * 2 * E, lane, ids + (size_t)m * k, w + (size_t)m * k);
+  int id; float wv;
+  route_row<SIG>(a, logits + (size_t)m * ld, sm_p + (size_t)warp * a.E, rs[warp], RouteGroup{0, 1, 0}, lane, id, wv);
+  if (lane < a.k) { ids[(size_t)m * a.k + lane] = id; w[(size_t)m * a.k + lane] = wv; }
 }
 
 __global__ void build_pairs_kernel(const int32_t* __restrict__ ids, const float* __restrict__ w, int M, int K, const uint8_t* const* __restrict__ tab,
@@ -90,15 +85,15 @@ static inline int grid_for(hb_ctx* ctx, size_t n, int per_block) {
 
 int hbk_route_softmax_topk(hb_ctx* ctx, const float* logits, int ld, int M, int E, int k, int renorm, int logits_bf16, int32_t* ids, float* w,
                            cudaStream_t st, bool pdl) {
-  const int warps = 4;
-  return hb_launch(ctx, "router_softmax", pdl, router_softmax_kernel, dim3((M + warps - 1) / warps), dim3(warps * 32), (size_t)warps * E * 4, st,
-                   logits, ld, M, E, k, renorm, logits_bf16, ids, w);
+  const RouteArgs a{1, E, k, renorm, logits_bf16, nullptr, 1.f};
+  return hb_launch(ctx, "router_softmax", pdl, router_kernel<false>, dim3((M + kRouterWarps - 1) / kRouterWarps), dim3(kRouterWarps * 32),
+                   (size_t)kRouterWarps * E * 4, st, a, logits, ld, M, ids, w);
 }
 int hbk_route_sigmoid_topk(hb_ctx* ctx, const float* logits, const float* bias, int M, int E, int k, float scale, int32_t* ids, float* w,
                            cudaStream_t st, bool pdl) {
-  const int warps = 4;
-  return hb_launch(ctx, "router_sigmoid", pdl, router_sigmoid_kernel, dim3((M + warps - 1) / warps), dim3(warps * 32), (size_t)warps * 2 * E * 4, st,
-                   logits, bias, M, E, k, scale, ids, w);
+  const RouteArgs a{2, E, k, 0, 0, bias, scale};
+  return hb_launch(ctx, "router_sigmoid", pdl, router_kernel<true>, dim3((M + kRouterWarps - 1) / kRouterWarps), dim3(kRouterWarps * 32),
+                   (size_t)kRouterWarps * E * 4, st, a, logits, E, M, ids, w);
 }
 int hbk_build_pairs(hb_ctx* ctx, const int32_t* ids, const float* w, int M, int K, const uint8_t* const* tab, int li, int E, hb_moe_pair* pairs,
                     cudaStream_t st, bool pdl) {

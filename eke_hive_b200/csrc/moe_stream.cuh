@@ -10,7 +10,7 @@ namespace hb {
 constexpr int kGroupRows = 8;         // activation rows per group = columns of one m16n8k16 tile
 constexpr int kSlice = 256;           // K elements per consumer warp
 constexpr int kMaxStages = 8;
-constexpr int kGroupThreads = 1024;
+constexpr int kGroupThreads = 512;    // grouping kernels
 
 struct Group { const uint8_t* rec; int start; int n; };
 static_assert(sizeof(Group) == 16, "Group layout");

@@ -1,99 +1,137 @@
-// Per-row routing by one warp, shared by the stand-alone router kernels (k_router.cu) and the fused route + group kernel
-// (k_moe_decode.cu).  The exp is the portable polynomial form, sums are taken per lane (e = lane, lane+32, …) and then by a
-// 16,8,4,2,1 butterfly, the k picks are summed in pick order — the CPU oracle does the same operations in the same order, so
-// ids and weights agree with it to the bit.
+// Per-row routing by a group of W warps, shared by the stand-alone router kernels (k_router.cu), the fused route + group kernel
+// (k_moe_decode.cu) and the expert-parallel route + push kernel (k_ep.cu).  The exp is the portable polynomial form, sums are taken
+// per lane of one warp (e = lane, lane+32, …) and then by a 16,8,4,2,1 butterfly, the k picks are summed in pick order — the CPU
+// oracle does the same operations in the same order, so ids and weights agree with it to the bit.
+//
+// What bounds routing in a decode step is the length of one warp's instruction stream: it runs once, a warp on its own issues an
+// instruction every 6-9 clocks of straight-line code, and a row of 512 experts in one warp took 9000 clocks (16 rows 14500, eight
+// rows of the sigmoid router 27000).  So the scores of a row are worked out by all warps of its group, in loops that are short, and the
+// picks are not k dependent rounds over all scores: the k-th largest of the 32 column maxima (column = e mod 32) is a bound that at
+// least k experts reach, the dozen or so that reach it are listed, and each counts how many of them come before it.
 #pragma once
 #include "hb_common.cuh"
 
 namespace hb {
 
-// (value, id) maximum with ties to the smaller id, over the warp
-__device__ __forceinline__ void warp_argmax(float& best, int& bid) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bid, o);
-    if (ob > best || (ob == best && oi < bid)) { best = ob; bid = oi; }
+constexpr int kRouteCand = 64;                                            // longer lists (long runs of equal scores) fall back to k rounds
+struct RouteShare { uint2 cand[kRouteCand]; uint2 pick[16]; uint32_t red[16]; uint32_t bound; int n; };   // one per row group, in shared memory
+struct RouteGroup { int warp, W, bar; };                                  // warp within the group, warps of the group, its named barrier
+
+struct RouteArgs {                                                        // of one call; kind: 1 softmax, 2 sigmoid + bias
+  int kind, E, k, renorm, logits_bf16; const float* bias; float scale;
+};
+
+__device__ __forceinline__ void route_sync(const RouteGroup& g) {
+  if (g.W == 1) __syncwarp();
+  else named_bar_sync(g.bar, 32 * g.W);
+}
+// Scores as unsigned numbers in the same order, 0 = not selectable.  Softmax: a non-negative float orders like its bits, NaN and the
+// -1 of a taken expert give 0.  Sigmoid: any finite sum of score and bias (+0 folds -0 into it, as a comparison would), NaN and the
+// -inf of a taken expert give 0.
+template <bool SIG>
+__device__ __forceinline__ uint32_t route_key(float v) {
+  if (!SIG) return v >= 0.f ? __float_as_uint(v) + 1u : 0u;
+  const uint32_t u = __float_as_uint(__fadd_rn(v, 0.f));
+  return v > -INFINITY ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;
+}
+__device__ __forceinline__ float route_max(float v, const RouteGroup& g, uint32_t* red, int lane) {   // of the group; v is not NaN
+  const uint32_t u = __float_as_uint(v);
+  uint32_t o = __reduce_max_sync(0xffffffffu, (u & 0x80000000u) ? ~u : (u | 0x80000000u));
+  if (g.W > 1) {
+    if (lane == 0) red[g.warp] = o;
+    route_sync(g);
+    o = __reduce_max_sync(0xffffffffu, lane < g.W ? red[lane] : 0u);
   }
+  return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o);
 }
 
-// Softmax top-k of one row.  p: E floats of shared memory owned by this warp.  Lanes 0..k-1 write ids[lane], w[lane].
-__device__ __forceinline__ void route_softmax_row(const float* __restrict__ lr, int E, int k, int renorm, int logits_bf16, float* p, int lane,
-                                                  int32_t* __restrict__ ids, float* __restrict__ w) {
-  float mx = -INFINITY;
-  for (int e = lane; e < E; e += 32) {
-    const float v = logits_bf16 ? bf16r(lr[e]) : lr[e];
-    p[e] = v;
-    mx = fmaxf(mx, v);
-  }
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+// One row (logits lr) by the whole group.  p: E floats of shared memory and rs belong to the group.  Lane l < k of the group's warp 0
+// gets pick l in (id, w); the other warps and lanes get nothing.  All warps of the group call it; it ends in step (a group may go on
+// to its next row).
+template <bool SIG>
+__device__ __forceinline__ void route_row(const RouteArgs& a, const float* __restrict__ lr, float* p, RouteShare& rs, const RouteGroup& g, int lane, int& id,
+                                          float& w) {
+  const int t = g.warp * 32 + lane, T = g.W * 32;
   float sum = 0.f;
-  for (int e = lane; e < E; e += 32) {
-    const float v = exp_portable(__fsub_rn(p[e], mx));
-    p[e] = v;
-    sum = __fadd_rn(sum, v);
-  }
-  for (int o = 16; o > 0; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
-  const float inv = __fdiv_rn(1.f, sum);
-  __syncwarp();
-  float my_w = 0.f, tot = 0.f;
-  int my_id = 0;
-  for (int r = 0; r < k; ++r) {
-    float best = -1.f;
-    int bid = 0x7fffffff;
-    for (int e = lane; e < E; e += 32) {
-      const float v = p[e];
-      if (v >= 0.f && v > best) { best = v; bid = e; }      // ascending e per lane: the first (smaller) id keeps a tie
+  if (!SIG) {
+    float mx = -INFINITY;
+#pragma unroll 4
+    for (int e = t; e < a.E; e += T) {
+      const float v = a.logits_bf16 ? bf16r(lr[e]) : lr[e];
+      p[e] = v;
+      mx = fmaxf(mx, v);
     }
-    warp_argmax(best, bid);
-    const float sw = __fmul_rn(best, inv);
-    tot = __fadd_rn(tot, sw);
-    if (lane == r) { my_id = bid; my_w = sw; }
-    if (bid != 0x7fffffff && (bid & 31) == lane) p[bid] = -1.f;
-    __syncwarp();
-  }
-  if (lane < k) {
-    const float sc = renorm ? __fdiv_rn(1.f, tot) : 1.f;
-    ids[lane] = my_id;
-    w[lane] = __fmul_rn(my_w, sc);
-  }
-}
-
-// Sigmoid top-k of one row: s = sigmoid(logit), pick k maxima of s + bias (first maximum = smaller id), w = s/(Σs + 1e-20)·scale
-// with Σ in pick order.  sc: 2·E floats of shared memory owned by this warp.
-__device__ __forceinline__ void route_sigmoid_row(const float* __restrict__ lr, const float* __restrict__ bias, int E, int k, float scale, float* sc,
-                                                  int lane, int32_t* __restrict__ ids, float* __restrict__ w) {
-  float* s = sc;
-  float* c = sc + E;
-  for (int e = lane; e < E; e += 32) {
-    const float v = sigmoid_portable(lr[e]);
-    s[e] = v;
-    c[e] = bias ? __fadd_rn(v, bias[e]) : v;
-  }
-  __syncwarp();
-  float my_s = 0.f, sum = 0.f;
-  int my_id = 0;
-  for (int j = 0; j < k; ++j) {
-    float best = -INFINITY;
-    int bid = 0x7fffffff;
-    for (int e = lane; e < E; e += 32) {
-      const float v = c[e];
-      if (v > best) { best = v; bid = e; }
+    mx = route_max(mx, g, rs.red, lane);
+#pragma unroll 2
+    for (int e = t; e < a.E; e += T) p[e] = exp_portable(__fsub_rn(p[e], mx));
+  } else {
+#pragma unroll 2
+    for (int e = t; e < a.E; e += T) {
+      const float b = a.bias ? a.bias[e] : 0.f;                           // a score is positive: + 0 leaves it as it is
+      p[e] = __fadd_rn(sigmoid_portable(lr[e]), b);
     }
-    warp_argmax(best, bid);
-    if (bid == 0x7fffffff) bid = 0;                           // every candidate already taken or NaN: keep a valid id
-    const float sv = s[bid];
-    sum = __fadd_rn(sum, sv);
-    if (lane == j) { my_id = bid; my_s = sv; }
-    __syncwarp();
-    if ((bid & 31) == lane) c[bid] = -INFINITY;
-    __syncwarp();
   }
-  if (lane < k) {
-    const float inv = __fdiv_rn(1.f, __fadd_rn(sum, 1e-20f));
-    ids[lane] = my_id;
-    w[lane] = __fmul_rn(__fmul_rn(my_s, inv), scale);
+  route_sync(g);
+  if (g.warp == 0) {
+    uint32_t best = 0u;
+#pragma unroll 8
+    for (int e = lane; e < a.E; e += 32) { const float v = p[e]; if (!SIG) sum = __fadd_rn(sum, v); best = max(best, route_key<SIG>(v)); }
+    if (!SIG) for (int o = 16; o > 0; o >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+    uint32_t bound = 0u;                                                  // the k-th largest distinct column maximum: no larger than the k-th largest one
+#pragma unroll 1
+    for (int r = 0; r < a.k; ++r) {
+      bound = __reduce_max_sync(0xffffffffu, best);
+      if (best == bound) best = 0u;
+    }
+    bound = max(bound, 1u);                                               // fewer than k distinct ones: every selectable expert is listed
+    if (lane == 0) { rs.bound = bound; rs.n = 0; }
+    if (lane < 16) rs.pick[lane] = make_uint2(0u, 0x7fffffffu);
   }
+  route_sync(g);
+  const uint32_t bound = rs.bound;
+#pragma unroll 2
+  for (int e = t; e < a.E; e += T) {
+    const uint32_t key = route_key<SIG>(p[e]);
+    if (key >= bound) { const int at = atomicAdd(&rs.n, 1); if (at < kRouteCand) rs.cand[at] = make_uint2(key, (uint32_t)e); }
+  }
+  route_sync(g);
+  if (g.warp == 0) {
+    const int n = rs.n;
+    if (n <= kRouteCand) {
+      for (int c = lane; c < n; c += 32) {
+        const uint2 me = rs.cand[c];
+        int r = 0;
+#pragma unroll 4
+        for (int i = 0; i < n; ++i) { const uint2 o = rs.cand[i]; r += o.x > me.x || (o.x == me.x && o.y < me.y); }   // the smaller id first among equals
+        if (r < a.k) rs.pick[r] = me;
+      }
+    } else {
+#pragma unroll 1
+      for (int r = 0; r < a.k; ++r) {
+        uint32_t mx = 0u, at = 0x7fffffffu;
+        for (int e = lane; e < a.E; e += 32) { const uint32_t key = route_key<SIG>(p[e]); if (key > mx) { mx = key; at = (uint32_t)e; } }
+        const uint32_t m = __reduce_max_sync(0xffffffffu, mx);
+        at = __reduce_min_sync(0xffffffffu, mx == m ? at : 0x7fffffffu);
+        if (m && (at & 31u) == (uint32_t)lane) p[at] = SIG ? -INFINITY : -1.f;
+        if (lane == 0) rs.pick[r] = make_uint2(m, m ? at : 0x7fffffffu);
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    const uint2 mine = rs.pick[lane & 15];
+    id = (int)mine.y;
+    float s, tot = 0.f;
+    if (!SIG) s = __fmul_rn(mine.x ? __uint_as_float(mine.x - 1u) : -1.f, __fdiv_rn(1.f, sum));
+    else {
+      if (id == 0x7fffffff) id = 0;                                       // nothing left to pick (NaN): keep a valid id
+      s = sigmoid_portable(lr[id]);
+    }
+#pragma unroll 4
+    for (int r = 0; r < a.k; ++r) tot = __fadd_rn(tot, __shfl_sync(0xffffffffu, s, r));
+    if (!SIG) w = __fmul_rn(s, a.renorm ? __fdiv_rn(1.f, tot) : 1.f);
+    else w = __fmul_rn(__fmul_rn(s, __fdiv_rn(1.f, __fadd_rn(tot, 1e-20f))), a.scale);
+  }
+  route_sync(g);                                                          // p and rs are free for the group's next row
 }
 
 }  // namespace hb

@@ -70,3 +70,25 @@ def test_zipf_biased_routing_matches(E, oracle):
     ids, w = E.router_softmax_topk(torch.from_numpy(lg).cuda(), 8, True, True)
     i0, w0 = oracle.router_softmax_topk(lg, 8, True, True, 0)
     assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+
+
+@pytest.mark.parametrize("Ex", [16, 31, 255, 256, 257, 511, 512, 513, 1023, 1024])
+def test_router_register_widths(E, oracle, Ex):
+    """Every register width of the row routers at its edges (8, 16, 32 scores a lane), with whole groups of equal scores: ids and
+    weights are integers and fp32 results of the same operations in the same order, so they are compared bit for bit."""
+    import torch
+    rng = np.random.default_rng(Ex)
+    k = 16
+    lg = (np.round(rng.normal(0, 1, (9, Ex)) * 4) / 4).astype(np.float32)
+    lg[1] = 0.25                                                  # all equal: the first k ids
+    lg[2] = -np.inf; lg[2, Ex // 2] = 1.0                         # one score far above the others, which all clamp to the same exp
+    for renorm in (True, False):
+        ids, w = E.router_softmax_topk(torch.from_numpy(lg).cuda(), k, renorm, False)
+        i0, w0 = oracle.router_softmax_topk(lg, k, renorm, False, 0)
+        assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+    lg[2] = 0.5
+    bias = (np.round(rng.normal(0, 1, Ex) * 2) / 2).astype(np.float32)     # negative sums of score and bias among them
+    for b in (bias, None):
+        ids, w = E.router_topk(torch.from_numpy(lg).cuda(), None if b is None else torch.from_numpy(b).cuda(), k, 2.5)
+        i0, w0 = oracle.router_sigmoid_topk(lg, b, k, 2.5, 0)
+        assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
