@@ -32,6 +32,7 @@ struct hb_ctx {
   // streaming down kernels (one per split-K width): whether the planned number of CTAs per SM is really resident, i.e. whether the
   // CTAs may meet inside the kernel (k_moe_decode.cu)
   const void* down_fn[8] = {nullptr}; bool down_meet[8] = {false};
+  int dense_clusters[4] = {0};   // dense GEMV: clusters of 1, 2, 4, 8 CTAs that are resident at once (k_dense.cu)
   char err[512] = {0};
   // optional per-kernel timing (hb_profile_enable): a start/stop event pair around every launch, aggregated by hb_profile_read
   bool prof_on = false;
@@ -65,22 +66,34 @@ inline int hb_fail(hb_ctx* ctx, int code, const char* fmt, ...) {
 // Every kernel launch of the library goes through hb_launch: it counts the launch, converts a launch failure into a status
 // with a message, optionally asks for programmatic dependent launch (the kernel then calls griddep_wait() before touching its
 // inputs) and, when profiling is on, brackets the kernel with a CUDA event pair (PDL is then off so the pair times the kernel alone).
+// cluster > 1: thread-block clusters of that many CTAs along x.
 template <typename... KArgs, typename... Args>
-inline int hb_launch(hb_ctx* ctx, const char* what, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                     Args... args) {
+inline int hb_launch_cluster(hb_ctx* ctx, const char* what, bool pdl, int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                             Args... args) {
   const bool prof = ctx->prof_on && ctx->prof_n < hb_ctx::kProfMax;
   if (prof) cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n], st);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = (pdl && !ctx->prof_on && !(ctx->flags & HB_FLAG_NO_PDL)) ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr; cfg.numAttrs = 0;
+  if (pdl && !ctx->prof_on && !(ctx->flags & HB_FLAG_NO_PDL)) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster; attr[cfg.numAttrs].val.clusterDim.y = 1; attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   if (prof) { cudaEventRecord(ctx->prof_ev[2 * ctx->prof_n + 1], st); ctx->prof_name[ctx->prof_n++] = what; }
   ctx->launches++;
   if (e != cudaSuccess) return hb_fail(ctx, HB_ERR_CUDA, "launch %s: %s", what, cudaGetErrorString(e));
   return HB_OK;
+}
+template <typename... KArgs, typename... Args>
+inline int hb_launch(hb_ctx* ctx, const char* what, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                     Args... args) {
+  return hb_launch_cluster(ctx, what, pdl, 1, kernel, grid, block, smem, st, args...);
 }
 
 inline size_t hb_align256(size_t b) { return (b + 255) / 256 * 256; }

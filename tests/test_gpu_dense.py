@@ -117,3 +117,37 @@ def test_dense_argument_errors(E):
     with pytest.raises(E.HbError) as ei:
         E.dense_gemv(G, torch.zeros((1, 200), dtype=torch.bfloat16, device="cuda"), ws=torch.zeros(4096, dtype=torch.uint8, device="cuda"))
     assert ei.value.status == -2
+
+
+@pytest.mark.parametrize("fmt", ["nvfp4", "lb3", "lb2"])
+@pytest.mark.parametrize("N,K,M", [(1, 256, 9), (23, 768, 16), (2080, 5376, 13), (48, 10240, 16), (37, 20736, 7), (24, 41216, 16)])
+def test_dense_gemv_splits_and_tiles(E, oracle, fmt, N, K, M):
+    """The edges of the row and column split: one row, rows past the last whole strip, one and two column tiles, K split over 1 to 8
+    CTAs and over two launches, K that is not a multiple of 512.  Bound: products are exact in f16 (NVFP4) or 1024-offset f16 fields, so
+    what differs from the oracle is the order of fp32 sums; sqrt(K)·2^-23 of the largest partial sum stays below 2e-3 of the RMS here."""
+    import torch
+    rng = np.random.default_rng(N + K + M)
+    x = oracle.bf16r(rng.normal(0, 1, (M, K)).astype(np.float32))
+    if fmt == "nvfp4":
+        q, s, g = oracle.nvfp4_quantize(rng.normal(0, 0.02, (N, K)).astype(np.float32), search=False)
+        G = E.GMat(E.FMT_NVFP4, N, K, torch.from_numpy(q).cuda(), torch.from_numpy(s).cuda(), None, g)
+        ref = oracle.gemv_nvfp4(q, s, g, x)
+        U, refu = G, ref
+    else:
+        G, (q, s, zp) = _lb_mat(E, oracle, N, K, 3 if fmt == "lb3" else 2, N + K)
+        U, (qu, su, zu) = _lb_mat(E, oracle, N, K, 3 if fmt == "lb3" else 2, N + K + 1)
+        ref, refu = oracle.lb_gemv(q, s, zp, 3 if fmt == "lb3" else 2, x), oracle.lb_gemv(qu, su, zu, 3 if fmt == "lb3" else 2, x)
+    y = E.dense_gemv(G, bf16_tensor(x)).cpu().numpy()
+    rms = np.sqrt(np.mean(ref.astype(np.float64) ** 2))
+    assert np.max(np.abs(y - ref)) <= 2e-3 * rms
+    y1 = E.dense_gemv(G, bf16_tensor(x[M - 1:])).cpu().numpy()
+    assert y1.tobytes() == y[M - 1:].tobytes()                           # the last row of the second tile alone
+    act = E.dense_gemv_gu(G, U, bf16_tensor(x)).float().cpu().numpy()
+    refa = oracle.dense_act(ref, refu)
+    # sums in another order may put bf16 g, u, silu(g) and the product one step (2^-7 of the value) to the side each; silu passes a relative
+    # change of g on |1 + g·(1 - sigmoid(g))| times, which is above 1 for g far below zero
+    gd = ref.astype(np.float64)
+    amp = np.abs(1.0 + gd * (1.0 - 1.0 / (1.0 + np.exp(-gd))))
+    rmsa = np.sqrt(np.mean(refa.astype(np.float64) ** 2))
+    assert np.all(np.abs(act - refa) <= 2.0 ** -7 * (amp + 3.0) * np.abs(refa) + 5e-3 * rmsa)
+    E.context().check_device()
