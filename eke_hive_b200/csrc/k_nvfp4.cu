@@ -88,32 +88,54 @@ __global__ void __launch_bounds__(256) nvfp4_gemv_kernel(const uint8_t* __restri
 }
 
 // ---- fp32 → NVFP4 (the device rule of the reference's requant kernels: one global scale from the tensor's largest magnitude, block
-// scale = e4m3(block amax · gs / 6), code = e2m1(v · gs / scale); no per-block scale search).  Four lanes share a block of 16: a lane
-// loads ONE float4 (a warp reads 512 contiguous bytes), the block's amax is two shuffles away, the four lanes work out the same scale
-// and each turns its own four values into 16 bits of codes (a warp writes 64 contiguous bytes).
-// The source of four consecutive values: an fp32 matrix, or an FP8 (e4m3) matrix with one fp32 scale per row (value = fp8 · row scale,
+// scale = e4m3(block amax · gs / 6), code = e2m1(v · gs / scale); no per-block scale search).  Two lanes share a block of 16: a lane holds
+// eight values (32 bytes), the block's amax is one shuffle away, both lanes work out the same scale and each turns its own values into
+// 32 bits of codes.
+//
+// Two passes over the matrix, because the global scale comes first.  Both are bound by the memory stream once the arithmetic is out of
+// the way: with four values a lane, an IEEE division each and scalar conversions the second pass was bound by its instructions.  Now a
+// division by the block's scale is a product with its reciprocal and one residual step (see div_by), two codes come out of one
+// conversion, and the second pass walks the matrix from its end, where the first pass has just left it in L2.  Measured at 17408 x 5120
+// (fp32, 356 MB in, 50 MB out): largest magnitude 79 → 73 µs, encode 128 → 74 µs, the call 187 → 136 (5.6 TB/s of what both passes touch).
+// The source of eight consecutive values: an fp32 matrix, or an FP8 (e4m3) matrix with one fp32 scale per row (value = fp8 · row scale,
 // the reference's FP8ROW weights).
 struct SrcF32 {
   const float4* w4;
-  __device__ __forceinline__ float4 load(size_t i) const { return __ldg(w4 + i); }
+  __device__ __forceinline__ void load(size_t i, float (&v)[8]) const {
+    const float4 a = __ldg(w4 + 2 * i), b = __ldg(w4 + 2 * i + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
 };
 struct SrcFp8Row {
-  const uint32_t* w8; const float* row_scale; int K4;                       // K4 = K / 4 groups per row
-  __device__ __forceinline__ float4 load(size_t i) const {
-    const uint32_t u = __ldg(w8 + i);
-    const float sr = __ldg(row_scale + i / (size_t)K4);
-    return make_float4(__fmul_rn(e4m3_to_f32(u & 0xffu), sr), __fmul_rn(e4m3_to_f32((u >> 8) & 0xffu), sr), __fmul_rn(e4m3_to_f32((u >> 16) & 0xffu), sr),
-                       __fmul_rn(e4m3_to_f32(u >> 24), sr));
+  const uint32_t* w8; const float* row_scale; int K8;                       // K8 = K / 8 groups per row
+  __device__ __forceinline__ void load(size_t i, float (&v)[8]) const {
+    const float sr = __ldg(row_scale + i / (size_t)K8);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t u = __ldg(w8 + 2 * i + h);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[4 * h + j] = __fmul_rn(e4m3_to_f32((u >> (8 * j)) & 0xffu), sr);
+    }
   }
 };
+__device__ __forceinline__ float absmax8(const float (&v)[8]) {
+  return fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))), fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
+}
+constexpr int AM_UNROLL = 4;                                                // groups of eight a thread has in flight
 template <class SRC>
-__global__ void __launch_bounds__(256) tensor_absmax_kernel(const SRC src, size_t n4, float* __restrict__ amax) {
+__global__ void __launch_bounds__(256) tensor_absmax_kernel(const SRC src, size_t n8, float* __restrict__ amax) {
   __shared__ float part[8];
   float m = 0.f;
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
-    const float4 v = src.load(i);
-    m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+  const size_t step = (size_t)gridDim.x * 256;
+  size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  for (; i + (AM_UNROLL - 1) * step < n8; i += AM_UNROLL * step) {
+    float v[AM_UNROLL][8];
+#pragma unroll
+    for (int u = 0; u < AM_UNROLL; ++u) src.load(i + u * step, v[u]);
+#pragma unroll
+    for (int u = 0; u < AM_UNROLL; ++u) m = fmaxf(m, absmax8(v[u]));
   }
+  for (; i < n8; i += step) { float v[8]; src.load(i, v); m = fmaxf(m, absmax8(v)); }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
   __syncthreads();
@@ -123,29 +145,54 @@ __global__ void __launch_bounds__(256) tensor_absmax_kernel(const SRC src, size_
     if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));   // one atomic per block; magnitudes order like their bits
   }
 }
+// t / d rounded to nearest, r = 1 / d rounded to nearest: the quotient's first guess and one residual step give the correctly rounded
+// quotient as long as nothing under- or overflows (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990).  Here |t| ≤ 2688 and d ≥ 2^-9; where t is so small that the residual underflows, the quotient is far below half of the smallest
+// code either way.  The sign is t's own (a residual of zero would turn -0 into +0).
+__device__ __forceinline__ float div_by(float t, float d, float r) {
+  const float q = __fmul_rn(t, r);
+  return copysignf(__fmaf_rn(__fmaf_rn(-q, d, t), r, q), t);
+}
+__device__ __forceinline__ uint32_t cvt_f32x2_e2m1x2(float lo, float hi) {   // one byte: low nibble = lo
+  uint32_t out;
+  asm("{\n .reg .b8 b;\n cvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n mov.b32 %0, {b, 0, 0, 0};\n}" : "=r"(out) : "f"(lo), "f"(hi));
+  return out;
+}
+constexpr int ENC_UNROLL = 2;                                               // groups of eight a thread encodes, loaded together
 template <class SRC>
-__global__ void __launch_bounds__(256) nvfp4_encode_kernel(const SRC src, size_t n4, const float* __restrict__ amax, uint16_t* __restrict__ q16,
+__global__ void __launch_bounds__(256) nvfp4_encode_kernel(const SRC src, size_t n8, const float* __restrict__ amax, uint32_t* __restrict__ q32,
                                                            uint8_t* __restrict__ s, float* __restrict__ g_mul) {
   const float am = *amax;
   const bool live = am > 0.f;
   const float gs = live ? __fdiv_rn(448.f * 6.f, am) : 1.f;
   if (blockIdx.x == 0 && threadIdx.x == 0) *g_mul = live ? __fdiv_rn(am, 448.f * 6.f) : 1.f;
-  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;                   // four values per thread; n4 is a multiple of 4, whole quads stay in range together
-  if (i >= n4) return;
-  const float4 v = src.load(i);
-  float m = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-  const unsigned quad = 0xfu << (threadIdx.x & 28);
-  m = fmaxf(m, __shfl_xor_sync(quad, m, 1));
-  m = fmaxf(m, __shfl_xor_sync(quad, m, 2));
-  const __nv_fp8_storage_t sc = __nv_cvt_float_to_fp8(__fdiv_rn(__fmul_rn(m, gs), 6.f), __NV_SATFINITE, __NV_E4M3);
-  const float sd = e4m3_to_f32(sc);
-  if ((threadIdx.x & 3) == 0) s[i >> 2] = (uint8_t)sc;
-  const float f[4] = {v.x, v.y, v.z, v.w};
-  uint32_t c = 0;
+  const size_t i0 = ((size_t)gridDim.x - 1 - blockIdx.x) * (256 * ENC_UNROLL) + threadIdx.x;   // n8 is even: a pair of lanes stays in range together
+  float v[ENC_UNROLL][8];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    if (sd > 0.f) c |= ((uint32_t)__nv_cvt_float_to_fp4(__fdiv_rn(__fmul_rn(f[j], gs), sd), __NV_E2M1, cudaRoundNearest) & 0xFu) << (4 * j);
-  q16[i] = (uint16_t)c;
+  for (int u = 0; u < ENC_UNROLL; ++u) if (i0 + u * 256 < n8) src.load(i0 + u * 256, v[u]);
+#pragma unroll
+  for (int u = 0; u < ENC_UNROLL; ++u) {
+    const size_t i = i0 + u * 256;
+    if (i >= n8) return;
+    float m = absmax8(v[u]);
+    m = fmaxf(m, __shfl_xor_sync(3u << (threadIdx.x & 30), m, 1));
+    const __nv_fp8_storage_t sc =
+        __nv_cvt_float_to_fp8(gs < INFINITY ? div_by(__fmul_rn(m, gs), 6.f, 1.f / 6.f) : __fdiv_rn(__fmul_rn(m, gs), 6.f), __NV_SATFINITE, __NV_E4M3);
+    const float sd = e4m3_to_f32(sc);
+    if ((threadIdx.x & 1) == 0) s[i >> 1] = (uint8_t)sc;
+    uint32_t c = 0;
+    if (sd > 0.f && gs < INFINITY) {
+      const float r = __frcp_rn(sd);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        c |= cvt_f32x2_e2m1x2(div_by(__fmul_rn(v[u][2 * j], gs), sd, r), div_by(__fmul_rn(v[u][2 * j + 1], gs), sd, r)) << (8 * j);
+    } else if (sd > 0.f) {                                                  // a tensor so small that its scale overflows: infinities among the products
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        c |= cvt_f32x2_e2m1x2(__fdiv_rn(__fmul_rn(v[u][2 * j], gs), sd), __fdiv_rn(__fmul_rn(v[u][2 * j + 1], gs), sd)) << (8 * j);
+    }
+    q32[i] = c;
+  }
 }
 
 // ---- per-row dynamic NVFP4 quantisation of bf16 rows (the rule of the reference's activation quantiser: gx = amax / (6·448), block
@@ -266,20 +313,20 @@ int hbk_nvfp4_gemv(hb_ctx* ctx, const uint8_t* w, const uint8_t* s, float g, int
 }
 
 template <class SRC>
-static int quantize_from(hb_ctx* ctx, const SRC& src, size_t n4, uint8_t* q, uint8_t* s, float* g_mul, float* amax, cudaStream_t st) {
+static int quantize_from(hb_ctx* ctx, const SRC& src, size_t n8, uint8_t* q, uint8_t* s, float* g_mul, float* amax, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(amax, 0, 4, st);
   if (e != cudaSuccess) return hb_fail(ctx, HB_ERR_CUDA, "memset amax: %s", cudaGetErrorString(e));
-  size_t blocks = (n4 + 255) / 256, cap = (size_t)ctx->sm_count * 8;
-  int r = hb_launch(ctx, "tensor_absmax", false, tensor_absmax_kernel<SRC>, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, st, src, n4, amax);
+  size_t blocks = (n8 + 255) / 256, cap = (size_t)ctx->sm_count * 8;
+  int r = hb_launch(ctx, "tensor_absmax", false, tensor_absmax_kernel<SRC>, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), 0, st, src, n8, amax);
   if (r) return r;
-  return hb_launch(ctx, "nvfp4_encode", false, nvfp4_encode_kernel<SRC>, dim3((unsigned)blocks), dim3(256), 0, st, src, n4, (const float*)amax,
-                   reinterpret_cast<uint16_t*>(q), s, g_mul);
+  return hb_launch(ctx, "nvfp4_encode", false, nvfp4_encode_kernel<SRC>, dim3((unsigned)((blocks + ENC_UNROLL - 1) / ENC_UNROLL)), dim3(256), 0, st, src, n8, (const float*)amax,
+                   reinterpret_cast<uint32_t*>(q), s, g_mul);
 }
 int hbk_nvfp4_quantize(hb_ctx* ctx, const float* w, int N, int K, uint8_t* q, uint8_t* s, float* g_mul, float* amax, cudaStream_t st) {
-  return quantize_from(ctx, SrcF32{reinterpret_cast<const float4*>(w)}, (size_t)N * K / 4, q, s, g_mul, amax, st);   // K is a multiple of 16
+  return quantize_from(ctx, SrcF32{reinterpret_cast<const float4*>(w)}, (size_t)N * K / 8, q, s, g_mul, amax, st);   // K is a multiple of 16
 }
 int hbk_requant_nvfp4(hb_ctx* ctx, const uint8_t* w_fp8, const float* row_scale, int N, int K, uint8_t* q, uint8_t* s, float* g_mul, float* amax, cudaStream_t st) {
-  return quantize_from(ctx, SrcFp8Row{reinterpret_cast<const uint32_t*>(w_fp8), row_scale, K / 4}, (size_t)N * K / 4, q, s, g_mul, amax, st);
+  return quantize_from(ctx, SrcFp8Row{reinterpret_cast<const uint32_t*>(w_fp8), row_scale, K / 8}, (size_t)N * K / 8, q, s, g_mul, amax, st);
 }
 
 int hbk_quant_rows_scatter(hb_ctx* ctx, const void* x, int ld, int n, int K, const int* dest, int nd, uint8_t* q, uint8_t* s, float* g, cudaStream_t st,

@@ -143,3 +143,36 @@ def test_expert_dequant_bit_exact(E, oracle):
         ref = oracle.nvfp4_dequant_bf16(q, s, float(g[gi]))
         assert np.array_equal(bf16_bits_of(got), ref), name
 
+
+
+@pytest.mark.parametrize("N,K", [(1, 16), (3, 48), (37, 1040), (300, 4096), (1, 8192 * 16 + 16)])
+def test_quantize_bits_at_the_rounding_edges(E, oracle, N, K):
+    """The quantiser's codes, scales and global against the oracle, bit for bit, where a quotient that is not correctly rounded would
+    show: values exactly on the code thresholds times every block scale and one step to either side, blocks from full scale down to
+    the smallest scale and to none, and sizes at the edges of a thread's, a warp's and a block's share.  The largest magnitude is 2688·2^-7,
+    so that the products with the global scale (2^7) are exact and the thresholds are hit."""
+    import torch
+    rng = np.random.default_rng(N + K)
+    codes = oracle.e4m3_table()[1:0x7F].astype(np.float32)                    # every positive block scale
+    edges = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0, 6.0, 0.0, 1e-6], np.float32)
+    b = N * K // 16
+    sd = codes[rng.integers(0, codes.size, b)]
+    v = edges[rng.integers(0, edges.size, (b, 16))] * sd[:, None]
+    v = np.nextafter(v, np.choose(rng.integers(0, 3, v.shape), [v, np.float32(0.0), np.float32(np.inf)]), dtype=np.float32)   # on it, a step below, a step above
+    v = np.where(rng.integers(0, 3, v.shape) == 0, rng.uniform(0, 6, v.shape).astype(np.float32) * sd[:, None], v)
+    v[:, 0] = 6.0 * sd                                                        # the block's largest value: its scale is sd
+    if b > 2:
+        v[1] = 0.0
+        v[2] *= np.float32(2.0 ** -20)                                        # a block below the smallest scale
+    w = (np.minimum(np.abs(v), 2688.0) * rng.choice(np.array([-1, 1], np.float32), v.shape)).astype(np.float32) * np.float32(2.0 ** -7)
+    w[b // 2, 0] = 2688.0 * 2.0 ** -7
+    w = w.reshape(N, K)
+    q, s, g = E.nvfp4_quantize(torch.from_numpy(w).cuda())
+    q0, s0, g0 = oracle.nvfp4_quantize(w, search=False)
+    no_zero_sign = lambda c: np.where((c & 0xF) == 8, c & 0xF0, c) & np.where((c >> 4) == 8, 0x0F, 0xFF)   # -0: the converter keeps the sign, the numpy rule drops it
+    assert np.array_equal(s.cpu().numpy(), s0) and np.array_equal(no_zero_sign(q.cpu().numpy()), no_zero_sign(q0))
+    assert np.float32(g.item()).tobytes() == np.float32(g0).tobytes()
+    small = (w * np.float32(2.0 ** -130)).astype(np.float32)                  # the global scale overflows: everything saturates, nothing is NaN
+    q, s, g = E.nvfp4_quantize(torch.from_numpy(small).cuda())
+    q0, s0, g0 = oracle.nvfp4_quantize(small, search=False)
+    assert np.array_equal(s.cpu().numpy(), s0) and np.float32(g.item()).tobytes() == np.float32(g0).tobytes()
