@@ -141,6 +141,17 @@ __device__ __forceinline__ float exp_portable(float x) {
 __device__ __forceinline__ float sigmoid_portable(float x) { return __fdiv_rn(1.f, __fadd_rn(1.f, exp_portable(-x))); }
 __device__ __forceinline__ float silu_portable(float x) { return __fdiv_rn(x, __fadd_rn(1.f, exp_portable(-x))); }
 
+// One thread of a converged warp, and the warp's number as a value the compiler knows to be the same for all lanes.  Tensor-core, TMA and
+// bulk-copy instructions take their operands from uniform registers; a thread picked by `lane == 0` under a branch on threadIdx.x / 32 is
+// not known to be alone, and every such instruction then costs a loop that brings its operands over (measured: 134 clocks a tcgen05.mma
+// with nothing else on the SM, 280 beside busy warps; under elect.sync 35).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.b32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ int warp_uniform() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // ---- shared-memory barriers and bulk asynchronous copies (sm_90+ PTX, used here for sm_100a) ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

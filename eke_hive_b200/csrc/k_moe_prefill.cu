@@ -119,10 +119,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
   uint64_t* acc_empty = acc_full + 1;                                        // the epilogue has read them
   uint64_t* mma_done = acc_empty + 1;                                        // the issuing thread's last operation has retired
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < PF_ST; ++s) { mbar_init(&full[s], 128 + 1); mbar_init(&empty[s], 1); }   // full: 128 scale threads (scales are in tensor memory) + the TMA thread
-    mbar_init(acc_full, 1); mbar_init(acc_empty, 256); mbar_init(mma_done, 1);
+    for (int s = 0; s < PF_ST; ++s) { mbar_init(&full[s], 4 + 1); mbar_init(&empty[s], 1); }   // full: four scale warps (scales are in tensor memory; one arrival each) + the TMA thread
+    mbar_init(acc_full, 1); mbar_init(acc_empty, 8); mbar_init(mma_done, 1);
     mbar_fence_init();
   }
   if (warp == 4) { tmem_alloc(tmem_slot, PF_TMEM_COLS); tmem_relinquish(); }
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
 
   if (warp == 5) {
     // ------------------------------------------------------------------------------------------------ TMA: codes of both operands, one thread
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (long long w = blockIdx.x; w < work && ok; w += gridDim.x) {
@@ -231,13 +231,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
         tc_st32(sfc + 16, wb);
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&full[stage]);                                           // (the slab is not written again before every thread has arrived here: the MMAs wait for all)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full[stage]);                            // (the slab is not written again before every thread has arrived here: the MMAs wait for all)
         va = na; vb = nb; vc = nc; na = fa; nb = fb; nc = fc;
       }
     }
   } else if (warp == 4) {
     // ------------------------------------------------------------------------------------------------ MMA issue: one thread
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, tcount = 0;
       bool ok = true;
       for (long long w = blockIdx.x; w < work && ok; w += gridDim.x, ++tcount) {
@@ -294,7 +295,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
           tc_ld32(trow + 32 * c, rg);
           tc_ld32(trow + 128 + 32 * c, ru);
           tc_wait_ld();
-          if (c2 == 1) { tc_fence_before(); mbar_arrive(acc_empty); }       // the accumulators are read: the next tile may start
+          if (c2 == 1) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(acc_empty); }       // the accumulators are read: the next tile may start
           float y[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -315,7 +316,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
             uint32_t r[32];
             tc_ld32(trow + 128 * half + 64 * p2 + 32 * c2, r);
             tc_wait_ld();
-            if (p2 == 1 && c2 == 1) { tc_fence_before(); mbar_arrive(acc_empty); }
+            if (p2 == 1 && c2 == 1) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(acc_empty); }
             float y[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) y[i] = __uint_as_float(r[i]) * f0;
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) pf_gemm_kernel(const PfGemmArgs
           uint32_t r[32];
           tc_ld32(trow + 32 * c, r);
           tc_wait_ld();
-          if (c == 4 * half + 3) { tc_fence_before(); mbar_arrive(acc_empty); }
+          if (c == 4 * half + 3) { tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(acc_empty); }
 #pragma unroll
           for (int q = 0; q < 8; ++q)
             *reinterpret_cast<float4*>(mine + q * 16) = make_float4(__uint_as_float(r[4 * q]) * f0, __uint_as_float(r[4 * q + 1]) * f0,
@@ -566,7 +567,7 @@ size_t pf_carve(void* ws, int S, int K, int E, int H, int I, PfWs* w) {
   const size_t P = (size_t)S * K;
   PfWs t;
   t.hist = (int*)take((size_t)PLAN_MAX_CTAS * E * 4); t.n_slots = (int*)take(4); t.n_tiles = (int*)take(4);
-  t.tiles = (TileRef*)take((P / PF_BM + E) * sizeof(TileRef)); t.perm = (int*)take(P * 4); t.pos_of = (int*)take(P * 4);
+  t.tiles = (TileRef*)take((P / A16_BN_MIN + E) * sizeof(TileRef)); t.perm = (int*)take(P * 4); t.pos_of = (int*)take(P * 4);
   t.tmB = (CUtensorMap*)take((size_t)E * 6 * sizeof(CUtensorMap));
   t.y = (__nv_bfloat16*)take(P * I * 2); t.part = (__nv_bfloat16*)take(P * H * 2);
   t.xq_s = (uint8_t*)take(P * H / 2); t.xs_s = (uint8_t*)take(P * H / 16); t.xg_s = (float*)take(P * 4);
@@ -607,6 +608,12 @@ int a16_make_map(hb_ctx* ctx, CUtensorMap* m, const void* base, size_t row_len, 
   return HB_OK;
 }
 
+struct A16Kernel { void (*fn)(const A16Args, const CUtensorMap); size_t smem; int bn; };
+A16Kernel a16_kernel(int bn) {
+  return bn == 64 ? A16Kernel{a16_gemm_kernel<64>, (size_t)A16Cfg<64>::SMEM, 64} : bn == 128 ? A16Kernel{a16_gemm_kernel<128>, (size_t)A16Cfg<128>::SMEM, 128}
+                                                                                              : A16Kernel{a16_gemm_kernel<256>, (size_t)A16Cfg<256>::SMEM, 256};
+}
+
 // bf16 activations on the tensor cores: plan (tiles of ≤ 256 pairs) → slot-ordered copy of the rows → gate/up GEMM → down GEMM → sums.
 // The copy of the rows lives in the buffer of the per-pair down rows: the gate/up GEMM has read it before the down GEMM writes there.
 int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids, const float* w, int M, int K, const __nv_bfloat16* x, int H, int I, float limit,
@@ -635,7 +642,10 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
   };
   for (int s0 = 0; s0 < M; s0 += S) {
     const int n = M - s0 < S ? M - s0 : S, P = n * K;
-    PlanArgs pl{ids + (size_t)s0 * K, P, E, lt, A16_BN, 1, W.hist, W.perm, W.pos_of, W.tiles, W.n_tiles, W.n_slots,
+    // the tile size by the pairs an expert gets on average: runs a standard deviation or two above it still fit one tile, and an
+    // expert's weights are dequantised once per tile (39 pairs on average: 64 beats 128 beats 256; figures in pf_a16.cuh)
+    const A16Kernel gk = a16_kernel((long long)P <= 44ll * E ? 64 : (long long)P <= 100ll * E ? 128 : 256);
+    PlanArgs pl{ids + (size_t)s0 * K, P, E, lt, gk.bn, 1, W.hist, W.perm, W.pos_of, W.tiles, W.n_tiles, W.n_slots,
                 reinterpret_cast<unsigned int*>(ctx->dev_err) + kErrPlanMeet, ctx->dev_err};
     int plan_ctas = (P + 2047) / 2048;
     if (plan_ctas > PLAN_MAX_CTAS) plan_ctas = PLAN_MAX_CTAS;
@@ -647,11 +657,11 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
     A16Args a{};
     common(0, &a);
     a.off_w = (uint32_t)L.w1; a.off_s0 = (uint32_t)L.s1; a.off_s1 = (uint32_t)L.s3; a.row2 = (int)((L.w3 - L.w1) / (size_t)(H / 2)); a.out = W.y;
-    if ((r = hb_launch(ctx, "a16_gemm_gu", false, a16_gemm_kernel, dim3(grid), dim3(A16_THREADS), (size_t)A16_SMEM, st, a, tm_x))) return r;
+    if ((r = hb_launch(ctx, "a16_gemm_gu", false, gk.fn, dim3(grid), dim3(A16_THREADS), gk.smem, st, a, tm_x))) return r;
     A16Args d{};
     common(1, &d);
     d.off_w = (uint32_t)L.w2; d.off_s0 = (uint32_t)L.s2; d.off_s1 = (uint32_t)L.s2; d.row2 = 64; d.out = W.part;
-    if ((r = hb_launch(ctx, "a16_gemm_down", false, a16_gemm_kernel, dim3(grid), dim3(A16_THREADS), (size_t)A16_SMEM, st, d, tm_y))) return r;
+    if ((r = hb_launch(ctx, "a16_gemm_down", false, gk.fn, dim3(grid), dim3(A16_THREADS), gk.smem, st, d, tm_y))) return r;
     const __nv_bfloat16* sh = cmb ? reinterpret_cast<const __nv_bfloat16*>(cmb->shared) + (size_t)s0 * H : nullptr;
     if ((r = hb_launch(ctx, "pf_sum_pairs", false, pf_sum_pairs_kernel, dim3((unsigned)((n + SUM_ROWS - 1) / SUM_ROWS < ctx->sm_count * 8 ? (n + SUM_ROWS - 1) / SUM_ROWS : ctx->sm_count * 8)), dim3(256), 0, st,
                        (const __nv_bfloat16*)W.part, (const int*)W.pos_of, w + (size_t)s0 * K, n, K, H, cmb ? (float*)nullptr : out + (size_t)s0 * H, sh,
@@ -674,7 +684,8 @@ int hbk_moe_prefill_setup(hb_ctx* ctx) {
   HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(pf_gemm_kernel<PF_GU>), cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
   HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(pf_gemm_kernel<PF_DOWN>), cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
   HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(pf_peak_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, PF_STAGE + 2048));
-  HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(a16_gemm_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, A16_SMEM));
+  for (int bn : {64, 128, 256})
+    HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(a16_kernel(bn).fn), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a16_kernel(bn).smem));
   return HB_OK;
 }
 

@@ -9,14 +9,14 @@
 // the decode operators, sums are fp32.  Rounding points after the sums are the reference's (g, u → bf16 after the
 // global scale, y → bf16, down → bf16 before the routing weight).
 //
-// A work item is 256 weight rows (two A tiles of 128) × one tile of pairs; the two accumulators fill the CTA's tensor memory, so
-// the MMAs of the next item wait for the epilogue.  Per 64 k values an item moves 32 KB of activations and 8 KB of codes from L2 into
+// A work item is 256 weight rows (two A tiles of 128) × one tile of pairs; with tiles of 256 pairs the two accumulators fill the CTA's
+// tensor memory and the MMAs of the next item wait for the epilogue.  Per 64 k values an item moves 32 KB of activations and 8 KB of codes from L2 into
 // shared memory (with one A tile per item the activation stream alone ran into what the SMs can pull out of L2).
 //
-// Per CTA (persistent, one per SM, 26 warps): warp 9 (one thread) streams by TMA the raw code boxes of the weights (128 bytes × 64
-// rows, 256 k values per row, through the anchored tensor map of the decode path) and the activation boxes (64 values × 64 rows of
+// Per CTA (persistent, one per SM, 27 warps): warp 9 (one thread) streams by TMA the raw code boxes of the weights (128 bytes × 64
+// rows, 256 k values per row, through the anchored tensor map of the decode path), warp 26 the activation boxes (64 values × 64 rows of
 // bf16) of the tile; warps 10-25 (eight per A tile) turn a raw box into four operand tiles, fetching their row's block scales from
-// global memory a raw box ahead; warp 8 (one thread) issues the MMAs (128 × N × 16, four per A tile and step); warps 0-3 and 4-7 run
+// global memory a raw box ahead; warp 8 and warp 27 (one thread each) issue the MMAs of an A tile (128 × N × 16, four a step); warps 0-3 and 4-7 run
 // the epilogues of the two accumulators.  Gate/up: an A tile holds 64 gate and 64 up rows arranged so that lanes l and l + 16 of a
 // warp hold the gate and the up value of the same row of I — SwiGLU needs one exchange.  Every wait is bounded; a barrier gets one
 // arrival per warp, not per thread (arrivals on one barrier are taken one after the other).
@@ -25,20 +25,37 @@
 
 namespace hb {
 
-constexpr int A16_BN = 256;                     // pairs of a tile (MMA N), at most
-constexpr int A16_STA = 2, A16_STB = 3;         // operand rings: dequantised weight tiles, activation tiles
-constexpr int A16_A1 = 128 * 128;               // one A tile: 128 rows × 64 bf16
-constexpr int A16_A = 2 * A16_A1;               // both A tiles of a step
-constexpr int A16_B = A16_BN * 128;             // 256 rows × 64 bf16
-constexpr int A16_RAW = 2 * 128 * 128;          // raw codes of both A tiles: 128 rows × 128 bytes each (256 k values per row)
-constexpr int A16_SMEM = 1024 + A16_STA * A16_A + A16_STB * A16_B + 2 * A16_RAW + 1024;
-constexpr int A16_THREADS = 26 * 32;            // warps 0-3 and 4-7 epilogues of the two A tiles, 8 MMA issue, 9 TMA, 10-17 and 18-25 dequantisation
-constexpr int A16_W_MMA = 8, A16_W_TMA = 9, A16_W_DQ0 = 10, A16_DQ_THREADS = 512;
-constexpr int A16_TMEM_COLS = 512;              // the accumulators of the two A tiles, 256 columns each
-static_assert(A16_SMEM <= 227 * 1024, "shared memory");
+// Shared memory and tensor memory by the pairs a tile may have (MMA N).  An expert's run decides what bounds the kernel: with 256 pairs the
+// tensor pipe (an MMA of M = 128 takes max(47, N / 2) clocks, measured) and the activation stream; with a few dozen pairs — a prompt of a
+// couple of thousand tokens over 512 experts — the weights: an activation stage is then a quarter of the size, so there is room for a
+// deeper ring of raw codes (they come from HBM), and the sums leave room in tensor memory: the dequantised weights go there, as the A
+// operand, without touching shared memory (writing them to it and reading them back was what bounded small tiles: 1050 of 1600 clocks a
+// step with the MMAs waiting on it), and with ≤ 64 pairs the sums of two items, so the MMAs need not wait for the epilogue.  Measured for
+// 1999 rows of 512 experts (hidden 2048, intermediate 512, top-10: 39 pairs an expert), tiles of ≤ 256 in shared memory → ≤ 64 in tensor
+// memory, with the issuing threads elected: gate/up 440 → 375 µs, down 260 → 205 µs (routed part).
+template <int BN_>
+struct A16Cfg {
+  static constexpr int BN = BN_;                                     // pairs of a tile, at most
+  static constexpr bool AT = BN <= 128;                              // the dequantised weights sit in tensor memory (else: swizzled tiles in shared memory)
+  static constexpr int STA = AT ? 4 : 2;                             // operand rings: dequantised weight tiles, activation tiles
+  static constexpr int STB = BN <= 64 ? 8 : BN <= 128 ? 5 : 3;
+  static constexpr int RAWS = AT ? 4 : 2;                            // raw code slots (256 k values each)
+  static constexpr int NACC = BN <= 64 ? 2 : 1;                      // accumulator buffers of 2·BN columns
+  static constexpr int A1 = 128 * 128;                               // one A tile: 128 rows × 64 bf16; raw codes of 256 k values take as much
+  static constexpr int A = AT ? 0 : 2 * A1;                          // both A tiles of a step in shared memory
+  static constexpr int B = BN * 128;                                 // BN rows × 64 bf16
+  static constexpr int RAW = 2 * A1;                                 // raw codes of both A tiles: 128 rows × 128 bytes each (256 k values per row)
+  static constexpr int ACOL = NACC * 2 * BN;                         // tensor memory: accumulators, then stages of two A tiles of 32 columns (bf16 pairs)
+  static constexpr int SMEM = 1024 + STA * A + STB * B + RAWS * RAW + 1024;
+  static_assert(SMEM <= 227 * 1024 && ACOL + (AT ? STA * 64 : 0) <= 512, "shared memory, tensor memory");
+};
+constexpr int A16_BN_MAX = 256, A16_BN_MIN = 64;
+constexpr int A16_THREADS = 28 * 32;            // warps 0-3 and 4-7 epilogues of the two A tiles, 8 and 27 their MMAs, 9 raw codes, 10-17 and 18-25 dequantisation, 26 activations
+constexpr int A16_W_MMA = 8, A16_W_TMA = 9, A16_W_DQ0 = 10, A16_W_ACT = 26, A16_W_MMA1 = 27, A16_DQ_THREADS = 512;
+constexpr int A16_TMEM_COLS = 512;
 
 struct A16Args {
-  const TileRef* tiles; const int* n_tiles;     // tiles of ≤ A16_BN consecutive slots of one expert's run of the sorted pairs
+  const TileRef* tiles; const int* n_tiles;     // tiles of ≤ BN consecutive slots of one expert's run of the sorted pairs
   const int* perm;                              // pair of a slot (the down pass writes its rows by pair)
   const uint8_t* const* tab;                    // expert records of the layer
   int down;                                     // 0: gate/up (out = y bf16 [slot, I]); 1: down (out = bf16 [pair, H])
@@ -58,6 +75,13 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+__device__ __forceinline__ void tc_mma_f16_at(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {   // A in tensor memory
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
 // two f16 values (exactly representable in bf16) → bf16x2, element order kept
@@ -118,30 +142,32 @@ __device__ long long g_a16_trace[2 * 256 * 16];   // gate/up launch, down launch
 #define A16_PUT(slot, v) do { } while (0)
 #endif
 
+template <int BN>
 __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args a, const __grid_constant__ CUtensorMap tmB) {
+  using C = A16Cfg<BN>;
   extern __shared__ uint8_t a16_raw[];
   const uint32_t raw0 = smem_u32(a16_raw), base = (raw0 + 1023u) & ~1023u;
   uint8_t* sm = a16_raw + (base - raw0);
   uint8_t* smA = sm;                                   // [STA][2 A tiles][16 KB]
-  uint8_t* smB = smA + A16_STA * A16_A;                // [STB][32 KB]
-  uint8_t* smR = smB + A16_STB * A16_B;                // [2][2 A tiles][16 KB] raw codes
-  uint64_t* fullA = reinterpret_cast<uint64_t*>(smR + 2 * A16_RAW);
-  uint64_t* emptyA = fullA + A16_STA;
-  uint64_t* fullB = emptyA + A16_STA;
-  uint64_t* emptyB = fullB + A16_STB;
-  uint64_t* fullR = emptyB + A16_STB;
-  uint64_t* emptyR = fullR + 2;
-  uint64_t* acc_full = emptyR + 2;
-  uint64_t* acc_empty = acc_full + 1;
-  uint64_t* mma_done = acc_empty + 1;
+  uint8_t* smB = smA + C::STA * C::A;                // [STB][32 KB]
+  uint8_t* smR = smB + C::STB * C::B;                // [RAWS][2 A tiles][16 KB] raw codes
+  uint64_t* fullA = reinterpret_cast<uint64_t*>(smR + C::RAWS * C::RAW);
+  uint64_t* emptyA = fullA + C::STA;
+  uint64_t* fullB = emptyA + C::STA;
+  uint64_t* emptyB = fullB + C::STB;
+  uint64_t* fullR = emptyB + C::STB;
+  uint64_t* emptyR = fullR + C::RAWS;
+  uint64_t* acc_full = emptyR + C::RAWS;                // [NACC]
+  uint64_t* acc_empty = acc_full + C::NACC;             // [NACC]
+  uint64_t* mma_done = acc_empty + C::NACC;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < A16_STA; ++s) { mbar_init(&fullA[s], A16_DQ_THREADS / 32); mbar_init(&emptyA[s], 1); }   // one arrival per dequantisation warp
-    for (int s = 0; s < A16_STB; ++s) { mbar_init(&fullB[s], 1); mbar_init(&emptyB[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&fullR[s], 1); mbar_init(&emptyR[s], A16_DQ_THREADS / 32); }
-    mbar_init(acc_full, 1); mbar_init(acc_empty, 8);
-    mbar_init(mma_done, 1);
+    for (int s = 0; s < C::STA; ++s) { mbar_init(&fullA[s], A16_DQ_THREADS / 32); mbar_init(&emptyA[s], 2); }   // one arrival per dequantisation warp; one commit per issuing thread
+    for (int s = 0; s < C::STB; ++s) { mbar_init(&fullB[s], 1); mbar_init(&emptyB[s], 2); }
+    for (int s = 0; s < C::RAWS; ++s) { mbar_init(&fullR[s], 1); mbar_init(&emptyR[s], A16_DQ_THREADS / 32); }
+    for (int s = 0; s < C::NACC; ++s) { mbar_init(&acc_full[s], 2); mbar_init(&acc_empty[s], 8); }
+    mbar_init(mma_done, 2);
     mbar_fence_init();
   }
   if (warp == A16_W_MMA) { tmem_alloc(tmem_slot, A16_TMEM_COLS); tmem_relinquish(); }
@@ -155,9 +181,9 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
   const int nk = a.K >> 6;                                    // steps per item (a multiple of 4)
 
   if (warp == A16_W_TMA) {
-    // ------------------------------------------------------------------------------------------------ loads: one thread
-    if (lane == 0) {
-      uint32_t rit = 0, kit = 0, seen = 0u;
+    // ------------------------------------------------------------------------------------------------ raw code boxes: one thread
+    if (elect_one()) {
+      uint32_t rit = 0, seen = 0u;
       bool ok = true;
       [[maybe_unused]] long long tw = 0, t0 = clock64();
       const unsigned long long anchor = *a.anchor;
@@ -180,34 +206,45 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
         const CUtensorMap* map = a.maps + v;
         if (!((seen >> v) & 1u)) { tmap_acquire(map); seen |= 1u << v; }
         const int r0 = (int)row + 2 * t * arows;
-        const int nbox = (tl.rows + 63) >> 6;
         for (int rs = 0; rs < nk / 4 && ok; ++rs, ++rit) {
-          const uint32_t sl = rit & 1u;
-          A16_TIMED(tw, ok = mbar_wait(&emptyR[sl], ((rit >> 1) & 1u) ^ 1u, a.err, 0x1u));
+          const uint32_t sl = rit % C::RAWS;
+          A16_TIMED(tw, ok = mbar_wait(&emptyR[sl], ((rit / C::RAWS) & 1u) ^ 1u, a.err, 0x1u));
           if (!ok) break;
-          const uint32_t rb = smem_u32(smR + sl * A16_RAW);
-          mbar_expect_tx(&fullR[sl], A16_RAW);
+          const uint32_t rb = smem_u32(smR + sl * C::RAW);
+          mbar_expect_tx(&fullR[sl], C::RAW);
 #pragma unroll
           for (int uu = 0; uu < 2; ++uu) {
-            tma_load_2d(rb + uu * A16_A1, map, rs * 128, r0 + uu * arows, &fullR[sl]);
-            tma_load_2d(rb + uu * A16_A1 + A16_A1 / 2, map, rs * 128, r0 + uu * arows + a.row2, &fullR[sl]);
-          }
-          for (int kq = 0; kq < 4; ++kq, ++kit) {
-            const uint32_t sb = kit % A16_STB;
-            A16_TIMED(tw, ok = mbar_wait(&emptyB[sb], ((kit / A16_STB) & 1u) ^ 1u, a.err, 0x2u));
-            if (!ok) break;
-            const uint32_t bb = smem_u32(smB + sb * A16_B);
-            mbar_expect_tx(&fullB[sb], (uint32_t)nbox * 8192u);
-            for (int i = 0; i < nbox; ++i) tma_load_2d(bb + i * 8192, &tmB, (rs * 4 + kq) * 64, tl.slot0 + i * 64, &fullB[sb]);
+            tma_load_2d(rb + uu * C::A1, map, rs * 128, r0 + uu * arows, &fullR[sl]);
+            tma_load_2d(rb + uu * C::A1 + C::A1 / 2, map, rs * 128, r0 + uu * arows + a.row2, &fullR[sl]);
           }
         }
       }
       A16_PUT(0, tw); A16_PUT(1, clock64() - t0);
     }
-  } else if (warp >= A16_W_DQ0) {
+  } else if (warp == A16_W_ACT) {
+    // ------------------------------------------------------------------------------------------------ activation boxes: one thread (apart from the codes, whose ring
+    // must run ahead whatever the activation ring does)
+    if (elect_one()) {
+      uint32_t kit = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < n_items_all && ok; item += gridDim.x) {
+        const TileRef tl = a.tiles[item / nT];
+        const int nbox = (tl.rows + 63) >> 6;
+        for (int kb = 0; kb < nk; ++kb, ++kit) {
+          const uint32_t sb = kit % C::STB;
+          if (!(ok = mbar_wait(&emptyB[sb], ((kit / C::STB) & 1u) ^ 1u, a.err, 0x2u))) break;
+          const uint32_t bb = smem_u32(smB + sb * C::B);
+          mbar_expect_tx(&fullB[sb], (uint32_t)nbox * 8192u);
+          for (int i = 0; i < nbox; ++i) tma_load_2d(bb + i * 8192, &tmB, kb * 64, tl.slot0 + i * 64, &fullB[sb]);
+        }
+      }
+    }
+  } else if (warp >= A16_W_DQ0 && warp < A16_W_DQ0 + A16_DQ_THREADS / 32) {
     // ------------------------------------------------------------------------------------------------ dequantisation: thread (u, r, h) owns half a row
     // of A tile u in every step: A row r, k values [32 h, 32 h + 32) of the step's 64
-    const int dt = threadIdx.x - A16_W_DQ0 * 32, u = dt >> 8, r = (dt & 255) >> 1, h = dt & 1;
+    // (A in tensor memory: a warp reaches the lanes of quarter (warp index mod 4), a thread's lane there is its row)
+    const int dt = threadIdx.x - A16_W_DQ0 * 32, u = dt >> 8, r = C::AT ? (warp & 3) * 32 + lane : (dt & 255) >> 1, h = C::AT ? (dt >> 7) & 1 : dt & 1;
+    const uint32_t acol = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::ACOL + u * 32 + h * 16;
     int rr, srow; uint32_t soff;                               // raw row, row of the scale matrix inside the A tile, which scale matrix
     if (a.down) { rr = r; srow = r; soff = a.off_s0; }
     else {
@@ -229,11 +266,11 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
       for (int rs = 0; rs < nk / 4 && ok; ++rs, ++rit) {
         uint4 sc_next = sc;
         if (rs + 1 < nk / 4) sc_next = __ldg(reinterpret_cast<const uint4*>(srowp + (size_t)(rs + 1) * 16));
-        const uint32_t sl = rit & 1u;
-        if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&fullR[sl], (rit >> 1) & 1u, a.err, 0x4u));
+        const uint32_t sl = rit % C::RAWS;
+        if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&fullR[sl], (rit / C::RAWS) & 1u, a.err, 0x4u));
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
-        const uint8_t* rawrow = smR + sl * A16_RAW + u * A16_A1 + rr * 128;
+        const uint8_t* rawrow = smR + sl * C::RAW + u * C::A1 + rr * 128;
         const uint32_t scw[4] = {sc.x, sc.y, sc.z, sc.w};
 #pragma unroll
         for (int kq = 0; kq < 4; ++kq, ++kit) {
@@ -250,16 +287,24 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
           tc += clock64() - tl0;
 #endif
           // one lane waits for the slot and one lane announces the warp's rows
-          const uint32_t sa = kit % A16_STA;
-          if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&emptyA[sa], ((kit / A16_STA) & 1u) ^ 1u, a.err, 0x8u));
+          const uint32_t sa = kit % C::STA;
+          if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&emptyA[sa], ((kit / C::STA) & 1u) ^ 1u, a.err, 0x8u));
           ok = __shfl_sync(0xffffffffu, ok, 0);
           if (!ok) break;
-          uint8_t* arow = smA + sa * A16_A + u * A16_A1 + r * 128;
-          *reinterpret_cast<uint4*>(arow + (((h * 4 + 0) ^ (r & 7)) << 4)) = o0;
-          *reinterpret_cast<uint4*>(arow + (((h * 4 + 1) ^ (r & 7)) << 4)) = o1;
-          *reinterpret_cast<uint4*>(arow + (((h * 4 + 2) ^ (r & 7)) << 4)) = o2;
-          *reinterpret_cast<uint4*>(arow + (((h * 4 + 3) ^ (r & 7)) << 4)) = o3;
-          fence_proxy_async_smem();
+          if constexpr (C::AT) {
+            tc_fence_after();
+            const uint32_t w16[16] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w, o2.x, o2.y, o2.z, o2.w, o3.x, o3.y, o3.z, o3.w};
+            tc_st16(acol + sa * 64, w16);
+            tc_wait_st();
+            tc_fence_before();
+          } else {
+            uint8_t* arow = smA + sa * C::A + u * C::A1 + r * 128;
+            *reinterpret_cast<uint4*>(arow + (((h * 4 + 0) ^ (r & 7)) << 4)) = o0;
+            *reinterpret_cast<uint4*>(arow + (((h * 4 + 1) ^ (r & 7)) << 4)) = o1;
+            *reinterpret_cast<uint4*>(arow + (((h * 4 + 2) ^ (r & 7)) << 4)) = o2;
+            *reinterpret_cast<uint4*>(arow + (((h * 4 + 3) ^ (r & 7)) << 4)) = o3;
+            fence_proxy_async_smem();
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(&fullA[sa]);
         }
@@ -270,42 +315,53 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
       }
     }
     if (dt == 0) { A16_PUT(2, tw); A16_PUT(3, clock64() - t0); A16_PUT(4, tc); }
-  } else if (warp == A16_W_MMA) {
-    // ------------------------------------------------------------------------------------------------ MMA issue: one thread
-    if (lane == 0) {
-      uint32_t kit = 0, n_it = 0;
+  } else if (warp == A16_W_MMA || warp == A16_W_MMA1) {
+    // ------------------------------------------------------------------------------------------------ MMA issue: one thread per A tile (one thread for both spent a
+    // thousand clocks a step on its instructions alone, in the shadow of sixteen dequantising warps)
+    const uint32_t uu = warp == A16_W_MMA ? 0u : 1u;
+    if (elect_one()) {
+      // few instructions a step: they run one at a time, between those of four other warps
+      uint32_t n_it = 0, sa = 0, pa = 0, sb = 0, pb = 0;
       bool ok = true;
-      [[maybe_unused]] long long twa = 0, twb = 0, twe = 0, t0 = clock64();
+      [[maybe_unused]] long long twa = 0, twb = 0, twe = 0, t0 = clock64(), kit = 0;
+      const uint64_t ad0 = tc_desc_sw128(base + uu * C::A1), bd0 = tc_desc_sw128(base + C::STA * C::A);
       for (int item = blockIdx.x; item < n_items_all && ok; item += gridDim.x, ++n_it) {
         const int rows = a.tiles[item / nT].rows;
         const uint32_t N = (uint32_t)((rows + 15) & ~15);
         // kind::f16: D fp32 (bit 4), A and B bf16 (format 1 at bits 7 and 10), both K-major, N / 8 at bit 17, M / 16 at bit 24
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
-        if (n_it >= 1) A16_TIMED(twe, ok = mbar_wait(acc_empty, (n_it - 1u) & 1u, a.err, 0x10u));   // the epilogue has read the previous item's sums
+        const uint32_t buf = n_it % C::NACC, acc = tmem + buf * (2 * BN) + uu * BN;
+        if (n_it >= C::NACC) A16_TIMED(twe, ok = mbar_wait(&acc_empty[buf], (n_it / C::NACC - 1u) & 1u, a.err, 0x10u));   // the epilogue has read the buffer's previous sums
         if (!ok) break;
         tc_fence_after();
-        for (int kb = 0; kb < nk; ++kb, ++kit) {
-          const uint32_t sa = kit % A16_STA, sb = kit % A16_STB;
-          A16_TIMED(twb, ok = mbar_wait(&fullB[sb], (kit / A16_STB) & 1u, a.err, 0x40u));
+        uint32_t more = 0u;                                       // 0 for the item's first MMA: it overwrites the accumulator
+        for (int kb = 0; kb < nk; ++kb) {
+          A16_TIMED(twb, ok = mbar_wait(&fullB[sb], pb, a.err, 0x40u));
           if (!ok) break;
-          A16_TIMED(twa, ok = mbar_wait(&fullA[sa], (kit / A16_STA) & 1u, a.err, 0x20u));
+          A16_TIMED(twa, ok = mbar_wait(&fullA[sa], pa, a.err, 0x20u));
           if (!ok) break;
           tc_fence_after();
-          const uint64_t ad = tc_desc_sw128(base + sa * A16_A), bd = tc_desc_sw128(base + A16_STA * A16_A + sb * A16_B);
+          const uint64_t ad = ad0 + sa * (uint32_t)(C::A >> 4), bd = bd0 + sb * (uint32_t)(C::B >> 4);
+          const uint32_t at = tmem + C::ACOL + sa * 64 + uu * 32;
 #pragma unroll
-          for (uint32_t uu = 0; uu < 2; ++uu) {
-#pragma unroll
-            for (uint32_t j = 0; j < 4; ++j)
-              tc_mma_f16(tmem + uu * 256, ad + uu * (A16_A1 >> 4) + 2 * j, bd + 2 * j, idesc, (kb | (int)j) != 0 ? 1u : 0u);
+          for (uint32_t j = 0; j < 4; ++j) {
+            if constexpr (C::AT) tc_mma_f16_at(acc, at + 8 * j, bd + 2 * j, idesc, j ? 1u : more);
+            else tc_mma_f16(acc, ad + 2 * j, bd + 2 * j, idesc, j ? 1u : more);
           }
+          more = 1u;
           tc_commit(&emptyA[sa]);
           tc_commit(&emptyB[sb]);
+          if (++sa == C::STA) { sa = 0; pa ^= 1u; }
+          if (++sb == C::STB) { sb = 0; pb ^= 1u; }
+#ifdef HB_A16_TRACE
+          ++kit;
+#endif
         }
-        if (ok) tc_commit(acc_full);
+        if (ok) tc_commit(&acc_full[buf]);
       }
       tc_commit(mma_done);
       mbar_wait(mma_done, 0, a.err, 0x80u);
-      A16_PUT(5, twa); A16_PUT(6, twb); A16_PUT(7, twe); A16_PUT(8, clock64() - t0); A16_PUT(9, (long long)kit);
+      A16_PUT(5, twa); A16_PUT(6, twb); A16_PUT(7, twe); A16_PUT(8, clock64() - t0); A16_PUT(9, kit);
     }
   } else {
     // ------------------------------------------------------------------------------------------------ epilogues: warp 4 u + q reads lanes [32 q, 32 q + 32) of accumulator u
@@ -321,15 +377,16 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
       const float gsc = __ldg(reinterpret_cast<const float*>(rec + a.off_g) + (a.down ? 2 : lane < 16 ? 0 : 1));
       // down: the pairs (output rows) of the tile's columns, lane l those of columns 32 i + l — fetched while the MMAs run and handed
       // round by shuffles below
-      int my_pair[A16_BN / 32];
+      int my_pair[C::BN / 32];
 #pragma unroll
-      for (int i = 0; i < A16_BN / 32; ++i) my_pair[i] = a.down && 32 * i + lane < tl.rows ? __ldg(a.perm + tl.slot0 + 32 * i + lane) : 0;
-      A16_TIMED(tw, ok = mbar_wait(acc_full, n_it & 1u, a.err, 0x100u));
+      for (int i = 0; i < C::BN / 32; ++i) my_pair[i] = a.down && 32 * i + lane < tl.rows ? __ldg(a.perm + tl.slot0 + 32 * i + lane) : 0;
+      const uint32_t buf = n_it % C::NACC;
+      A16_TIMED(tw, ok = mbar_wait(&acc_full[buf], (n_it / C::NACC) & 1u, a.err, 0x100u));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + u * 256;
+      const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + buf * (2 * BN) + u * BN;
 #pragma unroll
-      for (int ci = 0; ci < A16_BN / 32; ++ci) {
+      for (int ci = 0; ci < C::BN / 32; ++ci) {
         const int c0 = 32 * ci;
         if (c0 >= tl.rows) break;
         uint32_t rg[32];
@@ -364,7 +421,7 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
     if (threadIdx.x == 0) { A16_PUT(10, tw); A16_PUT(11, clock64() - t0); A16_PUT(12, tld); A16_PUT(13, (long long)n_it); }
   }
