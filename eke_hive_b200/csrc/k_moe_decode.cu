@@ -31,10 +31,14 @@ struct GroupArgs {
   RouteArgs rt; const float* logits; int ld;
   int32_t* ids_out; float* w_out;
   uint32_t k_inv;       // ceil(2^32 / K): i / K is the high word of i · k_inv (i, K ≤ HB_MAX_PAIRS; not for K = 1)
-  int group_shift;      // log2 of the rows per group (≤ kGroupRows)
 };
 
-constexpr int kTcGuMinPairs = 40;                   // unpinned contexts: pairs per call from which gate/up runs on the tensor-memory kernel
+// Where the gate/up pass of an unpinned context runs on the tensor-memory kernel.  One GPU: from kTcGuMinWork = pairs · H · I on; below it the
+// kernel's start-up (tensor-memory allocation, work table, first boxes) costs what its faster stream saves.  Measured per layer, tensor
+// memory against register kernels: hidden 2048, intermediate 512, top-10 + shared: 1 row (11 pairs) 23.3 / 22.6 us, 2 rows 26.8 / 29.3,
+// 16 rows 64.6 / 76.4, 64 rows 137 / 169; hidden 4096, intermediate 1536, top-8 + shared: 1 row 36.4 / 38.0, 8 rows 45 / 52, 64 rows 150 / 196.
+constexpr long long kTcGuMinWork = 16ll << 20;
+constexpr int kTcGuMinPairs = 40;                   // expert parallel: this rank's share of the pairs
 
 // Sorts the pairs by expert: counts the pairs of every expert, scans the counts, places the pairs.  It sits alone on the critical path in
 // front of the two weight passes, so what bounds it is its chain of loads, instructions and block barriers: the counters are cleared
@@ -62,7 +66,7 @@ __device__ __forceinline__ void group_body(const GroupArgs& a) {
   const bool routed = ROUTE || a.ids != nullptr;
   const int MK = a.M * a.K;
   const int P = routed ? MK + (a.shared_rec ? a.M : 0) : a.n_pairs;
-  const int NK = routed ? a.E + 1 : P;                  // key space: expert id (E = the shared expert) or leader pair index
+  const int NK = routed ? a.E + 1 : P;                  // key space: 0 = the shared expert (its groups are the fullest: the kernels behind this one meet them first), then the experts; or leader pair index
   constexpr int nt = kGroupThreads, nw = kGroupWarps;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint8_t** recs = reinterpret_cast<const uint8_t**>(gsm);       // [P], list form only
@@ -84,7 +88,7 @@ __device__ __forceinline__ void group_body(const GroupArgs& a) {
   const uint8_t* rec0 = nullptr;                        // the record of the thread's first key
   if (ROUTE) {
     const int cta = CTAS > 1 ? (int)cluster_rank() : 0;
-    if (cta == 0 && k0 < k1) rec0 = k0 == a.E ? a.shared_rec : tab[k0];
+    if (cta == 0 && k0 < k1) rec0 = k0 == 0 ? a.shared_rec : tab[k0 - 1];
     if (CTAS > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     const int wlog = route_wlog(a.M), grp = warp >> wlog, groups = nw >> wlog;
     const RouteGroup rg{warp - (grp << wlog), 1 << wlog, 1 + grp};
@@ -108,7 +112,7 @@ __device__ __forceinline__ void group_body(const GroupArgs& a) {
       if (cta != 0) return;
     } else __syncthreads();
   } else if (routed) {
-    if (k0 < k1) rec0 = k0 == a.E ? a.shared_rec : tab[k0];
+    if (k0 < k1) rec0 = k0 == 0 ? a.shared_rec : tab[k0 - 1];
     for (int i = tid; i < MK; i += nt) {
       const int row = row_of(i);
       const size_t src = (size_t)row * a.ld_ids + (i - row * a.K);
@@ -128,23 +132,24 @@ __device__ __forceinline__ void group_body(const GroupArgs& a) {
     if (!routed) {
       const uint8_t* r = recs[i];
       if (r) { kk = (uint32_t)i; for (int j = 0; j < i; ++j) if (recs[j] == r) { kk = (uint32_t)j; break; } }   // the first pair with this record stands for it
-    } else if (i < MK) kk = key[i] < (uint32_t)a.E ? key[i] : ~0u;
+    } else if (i < MK) kk = key[i] < (uint32_t)a.E ? key[i] + 1u : ~0u;
     else {                                              // one pair of weight 1 per row for the shared expert
       const int row = i - MK;
-      kk = row >= a.sh_row0 && row < a.sh_row0 + a.sh_rows ? (uint32_t)a.E : ~0u;
+      kk = row >= a.sh_row0 && row < a.sh_row0 + a.sh_rows ? 0u : ~0u;
       a.ws.pw[i] = 1.f;
     }
     key[i] = kk == ~0u ? ~0u : kk << 16 | atomicAdd(&cnt[kk], 1u);
   }
   __syncthreads();
   // exclusive scan over the keys of (pairs, groups), 16 bits each (at most HB_MAX_PAIRS = 4096 of either)
-  auto rec_of = [&](int k) { return !routed ? recs[k] : k == k0 ? rec0 : k == a.E ? a.shared_rec : tab[k]; };
-  const int gs = a.group_shift, gm = (1 << gs) - 1;     // rows per group: 8 for the streaming gate/up kernel, 2 for the tensor-memory one
+  auto rec_of = [&](int k) { return !routed ? recs[k] : k == k0 ? rec0 : k == 0 ? a.shared_rec : tab[k - 1]; };
+  constexpr int gm = kGroupRows - 1;
+  static_assert((kGroupRows & gm) == 0, "a power of two");
   uint32_t mine = 0u;
   for (int k = k0; k < k1; ++k) {
     uint32_t c = cnt[k];
     if (c && !rec_of(k)) { c = 0u; cnt[k] = kNoRec; }   // an expert without a record: its pairs are skipped
-    mine += c | ((c + gm) >> gs) << 16;
+    mine += c | ((c + gm) / kGroupRows) << 16;
   }
   uint32_t incl = mine;
 #pragma unroll
@@ -207,7 +212,7 @@ __device__ __forceinline__ void moe_stream_roles(const StreamArgs& a) {
   uint64_t* redbar = empty + kMaxStages;                                                        // [NSLOT][WM]
   uint64_t* redfree = redbar + (kMaxStages + 1) * WM;                                           // [NSLOT]
   uint8_t* ring = smem + C::head(S);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], C::NW); }
     for (int s = 0; s < NSLOT * WM; ++s) mbar_init(&redbar[s], WK);
@@ -229,7 +234,7 @@ __device__ __forceinline__ void moe_stream_roles(const StreamArgs& a) {
 
   if (warp == C::NW) {
     // ---------------------------------------------------------------- producer
-    if (lane == 0) {
+    if (elect_one()) {
       int s = 0, issued = 0;
       uint32_t ph = 0;
       Group g = {nullptr, 0, 0};
@@ -607,22 +612,19 @@ int hbk_moe_decode_run(hb_ctx* ctx, const hbk_pair_src& src, const void* x, int 
   ga.tab = src.tab; ga.li = src.li; ga.E = src.E; ga.shared_rec = src.shared_rec; ga.ws = w;
   ga.ld_ids = src.ld_ids ? src.ld_ids : src.K; ga.sh_row0 = src.sh_row0; ga.sh_rows = src.sh_rows < 0 ? src.M : src.sh_rows;
   ga.wait_flags = src.wait_flags; ga.wait_n = src.wait_n; ga.wait_step = src.wait_step; ga.wait_err = ctx->dev_err;
-  // Which gate/up engine: a context may pin either (HB_FLAG_DECODE_MMA_SYNC / HB_FLAG_DECODE_TC_GU).  Unpinned, the tensor-memory
-  // kernel takes calls of kTcGuMinPairs pairs or more — below that its start-up (tensor-memory allocation, work table, first TMA
-  // boxes) costs more than its faster stream saves (measured: 30.6 vs 27.6 µs per layer at 11 pairs, 73 vs 81 µs at 176).
-  // Expert parallel (rows of all ranks, most pairs dead on this rank): what counts is this rank's share of the pairs, and with many
-  // gathered rows the digit planes of rows this rank has nothing for cost more than the faster stream saves (measured at 8 ranks ×
-  // 16 rows: 109 vs 99 µs per layer; at 4 ranks × 16 rows: 99 vs 103 µs; at 2 ranks: 101 vs 108 µs) — unpinned contexts take the
+  // Which gate/up engine: a context may pin either (HB_FLAG_DECODE_MMA_SYNC / HB_FLAG_DECODE_TC_GU); unpinned, the size of the call decides
+  // (kTcGuMinWork).  Expert parallel (rows of all ranks, most pairs dead on this rank): what counts is this rank's share of the pairs, and
+  // with many gathered rows the digit planes of rows this rank has nothing for cost more than the faster stream saves (measured at 8
+  // ranks × 16 rows: 109 vs 99 µs per layer; at 4 ranks × 16 rows: 99 vs 103 µs; at 2 ranks: 101 vs 108 µs) — unpinned contexts take the
   // tensor-memory kernel up to 64 gathered rows.
   bool tc_gu = false;
   if (routed && !src.ws_stream_only && src.tab && hbk_moe_decode_fast(H, I) && hbk_moe_dtc_supported(H, I) && hbk_moe_dtc_gu_fits(ctx, P, src.E, H, I) &&
       !(ctx->flags & (HB_FLAG_DECODE_MMA_SYNC | HB_FLAG_FUSED))) {
     const int ranks = red.ep ? red.ep->world : 1;
-    const int pairs_eff = (P > src.pairs_hint ? P : src.pairs_hint) / ranks;
-    const bool auto_tc = pairs_eff >= kTcGuMinPairs && (ranks == 1 || src.M <= 64);
+    const int pairs = P > src.pairs_hint ? P : src.pairs_hint;
+    const bool auto_tc = ranks == 1 ? (long long)pairs * H * I >= kTcGuMinWork : pairs / ranks >= kTcGuMinPairs && src.M <= 64;
     tc_gu = (ctx->flags & (HB_FLAG_DECODE_TC_GU | HB_FLAG_DECODE_TC)) || auto_tc;
   }
-  ga.group_shift = tc_gu ? 1 : 3;
   const int x_ld = src.x_ld ? src.x_ld : H;
   if (src.route && ga.ld_ids != src.K) return hb_fail(ctx, HB_ERR_INVALID, "moe_decode: in-kernel routing writes dense ids / w rows");
   ga.rt = RouteArgs{src.route, src.E, src.K, src.renorm, src.logits_bf16, src.bias, src.sig_scale};

@@ -11,7 +11,7 @@
 // Every product is exact; sums are fp32.  Rounding points after the products are the reference's (g, u → bf16 after the global
 // scale, y → bf16).
 //
-// Where it sits: the streaming path's grouping kernel (k_moe_decode.cu; asked for groups of ≤ 2 rows) → beside it `moe_xdig_kernel`
+// Where it sits: the streaming path's grouping kernel (k_moe_decode.cu; groups of ≤ 8 rows) → beside it `moe_xdig_kernel`
 // (one CTA per activation row: the row's digit planes) → `moe_dtc_layer_kernel` (this file) → the streaming down kernel, which
 // reads y as bf16 rows.  A whole-layer form of this kernel (down items fed by digit planes of y published slice by slice, sums after
 // the CTAs meet) was built first; it was slower than this chain and not run-to-run stable in its down phase, and is gone.
@@ -28,11 +28,14 @@
 
 namespace hb {
 
-constexpr int DT_ST = 10;                      // pipeline stages
+constexpr int DT_ST = 8;                       // pipeline stages
 constexpr int DT_A = 16384;                    // weight tile of a stage: 128 rows × 128 bytes (256 k values)
-constexpr int DT_B = 2048;                     // digit planes of a stage: 2 activation rows × 8 planes × 128 bytes (most experts of a decode batch get one
-                                               // or two rows, and a small slot leaves room for more stages)
-constexpr int DT_ROWS = DT_B / 1024;           // activation rows of a group
+// Activation rows of a group: up to 8 share one pass over an expert's weights.  Groups of two, what this kernel had first, are the same speed
+// where every expert gets one or two rows, and read a hot expert's record once per two rows: 160 experts under skewed routing, 8 / 16 /
+// 45 rows 66 / 106 / 265 us per layer against 45 / 62 / 118 now (512 evenly routed experts, 16 / 45 rows: 63.6 / 116 against 64.6 / 113).  An MMA of
+// 16 columns takes as long as one of 64 (47 clocks), and eight stages are enough: five to ten made no difference.
+constexpr int DT_ROWS = kGroupRows;
+constexpr int DT_B = DT_ROWS * 1024;           // digit planes of a stage: 8 planes × 128 bytes per activation row
 constexpr int DT_STAGE = DT_A + DT_B;
 constexpr int DT_RAWD = 3;                     // windows the scale fetch runs ahead of its use
 constexpr int DT_RAW = (DT_RAWD + 1) * 2048;   // ring of fetched scale rows: 128 rows × 16 bytes per window
@@ -187,17 +190,18 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mma_done + 1);
   DtEnt* tbl = reinterpret_cast<DtEnt*>(reinterpret_cast<uint8_t*>(full) + 1024);   // [DT_TBL] this CTA's work list
   uint16_t* tbl_row = reinterpret_cast<uint16_t*>(tbl + DT_TBL);                // [DT_TBL][DT_ROWS] activation rows of the item's group
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < DT_ST; ++s) { mbar_init(&full[s], 128 + 2); mbar_init(&empty[s], 1); }   // full: 128 scale threads + the two copy threads
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 128); }
+    // (one arrival per warp, not per thread: arrivals on one barrier are taken one after the other)
+    for (int s = 0; s < DT_ST; ++s) { mbar_init(&full[s], 4 + 2); mbar_init(&empty[s], 1); }   // full: four scale warps + the two copy threads
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
     mbar_init(mma_done, 1);
     mbar_fence_init();
   }
   if (warp == DT_W_MMA) { tmem_alloc(tmem_slot, DT_TMEM_COLS); tmem_relinquish(); }
   // the first variant of the tensor map (the only one when the pitch divides 4096) is made visible to the TMA thread before the
   // wait: the maps were stamped by an earlier launch that has completed
-  if (threadIdx.x == DT_W_TMA * 32) tmap_acquire(a.maps);
+  if (warp == DT_W_TMA) tmap_acquire(a.maps);                                  // by every lane: whichever of them is elected below
   griddep_wait();                                                               // the group list and the digit planes of the rows
   griddep_launch();
   const int nIT = (int)a.dIT.d, grid = (int)a.dG.d, c0 = (int)blockIdx.x;
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
 
   if (warp == DT_W_TMA) {
     // ------------------------------------------------------------------------------------------------ weight boxes: one thread
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, seen = 1u;                                                // variant 0: acquired in the prologue
       bool ok = true;
       [[maybe_unused]] long long tw = 0, t_begin = clock64();
@@ -260,23 +264,24 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
     }
   } else if (warp == DT_W_DIG) {
     // ------------------------------------------------------------------------------------------------ digit planes: one thread walks the items' stages in ring
-    // order — wait for the slot, announce the bytes, copy the 1 KB plane atoms of the group's one or two rows (a row's planes of
+    // order — wait for the slot, announce the bytes, copy the 1 KB plane atoms of the group's rows (a row's planes of
     // consecutive k windows are contiguous in global memory).  (In order, by one thread: a wait by parity tells apart only
     // neighbouring phases of a slot, so nobody may wait for a slot more than one ring cycle ahead.)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int ii = 0; ii < n_items && ok; ++ii) {
         const int n = ent_n(tbl[ii]);
-        const uint8_t* s0 = a.dw.xdig + (size_t)tbl_row[ii * DT_ROWS] * nkb * 1024;
-        const uint8_t* s1 = n > 1 ? a.dw.xdig + (size_t)tbl_row[ii * DT_ROWS + 1] * nkb * 1024 : nullptr;
+        const uint8_t* src[DT_ROWS];
+#pragma unroll
+        for (int c = 0; c < DT_ROWS; ++c) src[c] = a.dw.xdig + (size_t)tbl_row[ii * DT_ROWS + c] * nkb * 1024;
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const uint32_t stage = it % DT_ST;
           if (!(ok = mbar_wait(&empty[stage], ((it / DT_ST) & 1) ^ 1, a.err, 0x2u))) break;
           uint8_t* dst = sm + stage * DT_STAGE + DT_A;
           mbar_expect_tx(&full[stage], (uint32_t)n * 1024u);
-          bulk_g2s(dst, s0 + (size_t)kb * 1024, 1024, &full[stage]);
-          if (s1) bulk_g2s(dst + 1024, s1 + (size_t)kb * 1024, 1024, &full[stage]);
+#pragma unroll
+          for (int c = 0; c < DT_ROWS; ++c) if (c < n) bulk_g2s(dst + c * 1024, src[c] + (size_t)kb * 1024, 1024, &full[stage]);
         }
       }
     }
@@ -334,7 +339,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
         for (int qq = 0; qq < 4; ++qq) if (qq == q) w16[4 * j + qq] = vj[j];
       }
       // the previous stage's stores have had this long to land: announce it before anything below can wait
-      if (pend >= 0) { tc_wait_st(); tc_fence_before(); mbar_arrive(&full[pend]); pend = -1; }
+      if (pend >= 0) { tc_wait_st(); tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(&full[pend]); pend = -1; }
       DT_TIMED(tw, ok = mbar_wait(&empty[stage], ((it / DT_ST) & 1) ^ 1, a.err, 0x4u));   // the MMAs that read this stage's scale columns are done
       if (!ok) break;
       tc_fence_after();
@@ -342,18 +347,20 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
       pend = (int)stage;
       if (r == 0) DT_STAMP(it, 2);
     }
-    if (pend >= 0 && ok) { tc_wait_st(); tc_fence_before(); mbar_arrive(&full[pend]); }
+    if (pend >= 0 && ok) { tc_wait_st(); tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(&full[pend]); }
     pf_cp_wait<0>();
     if (r == 0) { DT_TRACE_PUT(5, tw); DT_TRACE_PUT(6, tg); }
   } else if (warp == DT_W_MMA) {
     // ------------------------------------------------------------------------------------------------ MMA issue: one thread
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       [[maybe_unused]] long long tf = 0, te = 0, t_begin = clock64();
-      // 128 × 16 × 64 per instruction: A and B e2m1 (format 1), both K-major, N / 8 at bit 17, ue4m3 scales, M / 16 at bit 24
-      constexpr uint32_t idesc = (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
       for (int ii = 0; ii < n_items && ok; ++ii) {
+        // 128 × N × 64 per instruction, N = the planes of the group's rows in 16s (an odd row's partner planes are whatever the slot held, in
+        // columns nobody reads): A and B e2m1 (format 1), both K-major, N / 8 at bit 17, ue4m3 scales, M / 16 at bit 24
+        const uint32_t N = (uint32_t)((ent_n(tbl[ii]) + 1) >> 1) * 16u;
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((128u >> 4) << 24);
         const uint32_t buf = (uint32_t)ii & 1u;
         if (ii >= 2) DT_TIMED(te, ok = mbar_wait(&acc_empty[buf], ((ii >> 1) - 1) & 1, a.err, 0x8u));
         if (!ok) break;
@@ -398,24 +405,25 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
       DT_TIMED(ta, ok = mbar_wait(&acc_full[set], (ii >> 1) & 1, a.err, 0x80u));
       if (!ok) break;
       tc_fence_after();
-      float val[DT_ROWS];
-      {
-        uint32_t rr[16];                                                         // two activation rows × eight planes
-        tc_ld16(trow, rr);
-        tc_wait_ld();
+      float gu[DT_ROWS];
 #pragma unroll
-        for (int h = 0; h < DT_ROWS; ++h) {
-          float acc = __uint_as_float(rr[8 * h]);
+      for (int c = 0; c < DT_ROWS; c += 2) {                                     // two activation rows × eight planes
+        if (c < n) {
+          uint32_t rr[16];
+          tc_ld16(trow + 8 * c, rr);
+          tc_wait_ld();
 #pragma unroll
-          for (int p = 1; p < 8; ++p) acc = __fmaf_rn(acc, 8.f, __uint_as_float(rr[8 * h + p]));
-          val[h] = acc;
+          for (int h = 0; h < 2; ++h) {
+            float acc = __uint_as_float(rr[8 * h]);
+#pragma unroll
+            for (int p = 1; p < 8; ++p) acc = __fmaf_rn(acc, 8.f, __uint_as_float(rr[8 * h + p]));
+            gu[c + h] = bf16r(acc * un[c + h] * gsc);
+          }
         }
       }
       tc_fence_before();
-      mbar_arrive(&acc_empty[set]);
-      float gu[DT_ROWS];
-#pragma unroll
-      for (int c = 0; c < DT_ROWS; ++c) gu[c] = c < n ? bf16r(val[c] * un[c] * gsc) : 0.f;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[set]);
       if (a.down) {
         // a pair's row of the down projection, bf16 (the routing weight is applied where the pairs are summed): 128 threads, 256 contiguous bytes
 #pragma unroll
@@ -430,7 +438,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
       named_bar_sync(bar_id, 128);
       float upv[DT_ROWS];
 #pragma unroll
-      for (int c = 0; c < DT_ROWS; ++c) upv[c] = (tl < 64 && c < n) ? ex[c * 64 + tl] : 0.f;
+      for (int c = 0; c < DT_ROWS; ++c) if (c < n) upv[c] = ex[c * 64 + (tl & 63)];
       named_bar_sync(bar_id, 128);                                               // the up values are read: the item after next may overwrite them
       if (tl < 64) {
         // y = bf16(silu(g)·u): 64 threads, 128 contiguous bytes per activation row
