@@ -316,7 +316,8 @@ size_t layer_carve(void* ws, int M, int K, int E, int H, int I, LayerWs* w) {
   t.tab1 = (const uint8_t**)take(256); t.ids1 = (int32_t*)take(pf ? (size_t)M * 4 : 0); t.w1 = (float*)take(pf ? (size_t)M * 4 : 0);
   t.sh32 = (float*)take(pf ? (size_t)M * H * 4 : 0); t.sh16 = take(pf ? (size_t)M * H * 2 : 0);
   if (w) *w = t;
-  return off;
+  const size_t one = pf ? hbk_moe_layer_a16_ws_bytes(M, K, E, H, I) : 0;     // the other way to run the layer starts at the same place
+  return off > one ? off : one;
 }
 }  // namespace
 
@@ -358,6 +359,9 @@ int hb_moe_layer(hb_ctx* ctx, const float* logits, int ld, int M, int E, int K, 
                   : hbk_route_softmax_topk(ctx, logits, ld, M, E, K, renorm, logits_bf16, ids_out, w_out, st, false);
   if (r) return r;
   hb_pf_combine cmb = {};
+  if (shared_rec && hbk_moe_layer_a16_takes(ctx, M, K, E, H, I))
+    return hbk_moe_layer_a16(ctx, rec_tab + (size_t)li * E, E, shared_rec, ids_out, w_out, M, K, x, H, I, limit, gate_col >= 0 ? logits : nullptr, ld,
+                             gate_col >= 0 ? gate_col : 0, out, ws, st);
   if (shared_rec) {
     if ((r = hbk_layer_prep(ctx, W.tab1, W.ids1, W.w1, M, shared_rec, st))) return r;
     if ((r = hb_moe_prefill(ctx, W.tab1, 0, 1, W.ids1, W.w1, M, 1, x, H, I, limit, W.sh32, W.op, M, stream, nullptr))) return r;

@@ -18,6 +18,11 @@ int hbk_a4_quant(hb_ctx* ctx, const void* x, int ld, int n, int K, uint8_t* q, u
 // device word holding the number of rows to do when that is smaller than n
 int hbk_quant_rows_scatter(hb_ctx* ctx, const void* x, int ld, int n, int K, const int* dest, int nd, uint8_t* q, uint8_t* s, float* g, cudaStream_t st,
                            const int* n_dev = nullptr);
+// a whole bf16-activation prefill layer behind the router, shared expert included (k_moe_prefill.cu)
+size_t hbk_moe_layer_a16_ws_bytes(int M, int K, int E, int H, int I);
+bool hbk_moe_layer_a16_takes(const hb_ctx* ctx, int M, int K, int E, int H, int I);
+int hbk_moe_layer_a16(hb_ctx* ctx, const uint8_t* const* lt, int E, const uint8_t* shared_rec, const int32_t* ids, const float* w, int M, int K, const void* x, int H,
+                      int I, float limit, const float* lg, int ld, int col, void* out, void* ws, cudaStream_t st);
 int hbk_nvfp4_setup(hb_ctx* ctx);
 
 int hbk_route_softmax_topk(hb_ctx* ctx, const float* logits, int ld, int M, int E, int k, int renorm, int logits_bf16, int32_t* ids, float* w,

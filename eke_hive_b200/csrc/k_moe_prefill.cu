@@ -491,10 +491,11 @@ __global__ void pf_tmaps_kernel(const __grid_constant__ PfMapSet tpl, const uint
 // ---- the sum over a row's pairs -----------------------------------------------------------------------------------------------------
 // out[row] = Σ_k part[row·K + k]·w[row, k], fp32 in k order, overwritten — or the shared-expert combine on top of it:
 // out = bf16(bf16(Σ) + bf16(bf16(sigmoid(bf16 gate logit))·shared)); lg == NULL: no gate.  A CTA takes whole rows: the row's weights
-// and which of its pairs contributed (pos_of ≥ 0) are looked up once per row, then every thread streams 8 columns at a time.
+// and which of its pairs contributed (pos_of ≥ 0) are looked up once per row, then every thread streams 8 columns at a time.  The list holds
+// Kp pairs a row, the first K of them routed; with Kp = K + 1 the last one is the shared expert's (cout wanted, shared == NULL).
 constexpr int SUM_ROWS = 4;              // rows a CTA of pf_sum_pairs_kernel works on at once
 __global__ void __launch_bounds__(256) pf_sum_pairs_kernel(const __nv_bfloat16* __restrict__ part, const int* __restrict__ pos_of, const float* __restrict__ w, int M,
-                                                           int K, int H, float* __restrict__ out, const __nv_bfloat16* __restrict__ shared,
+                                                           int K, int Kp, int H, float* __restrict__ out, const __nv_bfloat16* __restrict__ shared,
                                                            const float* __restrict__ lg, int ld, int col, __nv_bfloat16* __restrict__ cout) {
   __shared__ float wk[SUM_ROWS][32];
   __shared__ uint32_t live[SUM_ROWS];
@@ -504,7 +505,7 @@ __global__ void __launch_bounds__(256) pf_sum_pairs_kernel(const __nv_bfloat16* 
     const int nr = min(SUM_ROWS, M - m0);
     if ((int)threadIdx.x < nr * 32) {
       const int r = threadIdx.x >> 5, k = threadIdx.x & 31;
-      const bool on = k < K && pos_of[(size_t)(m0 + r) * K + k] >= 0;
+      const bool on = k < K && pos_of[(size_t)(m0 + r) * Kp + k] >= 0;
       wk[r][k] = k < K ? w[(size_t)(m0 + r) * K + k] : 0.f;
       const uint32_t mask = __ballot_sync(0xffffffffu, on);
       if (k == 0) {
@@ -521,7 +522,7 @@ __global__ void __launch_bounds__(256) pf_sum_pairs_kernel(const __nv_bfloat16* 
         uint4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (k0 + j < K && ((lv >> (k0 + j)) & 1u)) v[j] = __ldcs(reinterpret_cast<const uint4*>(part + ((size_t)m * K + k0 + j) * H + n));
+          if (k0 + j < K && ((lv >> (k0 + j)) & 1u)) v[j] = __ldcs(reinterpret_cast<const uint4*>(part + ((size_t)m * Kp + k0 + j) * H + n));
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (k0 + j >= K || !((lv >> (k0 + j)) & 1u)) continue;
@@ -537,7 +538,7 @@ __global__ void __launch_bounds__(256) pf_sum_pairs_kernel(const __nv_bfloat16* 
         *reinterpret_cast<float4*>(out + o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
       } else {
         const float gate = gate_s[r];
-        const uint4 sv = *reinterpret_cast<const uint4*>(shared + o);
+        const uint4 sv = shared ? *reinterpret_cast<const uint4*>(shared + o) : __ldcs(reinterpret_cast<const uint4*>(part + ((size_t)m * Kp + K) * H + n));
         const uint32_t su[4] = {sv.x, sv.y, sv.z, sv.w};
         float rr[8];
 #pragma unroll
@@ -550,6 +551,14 @@ __global__ void __launch_bounds__(256) pf_sum_pairs_kernel(const __nv_bfloat16* 
     }
     __syncthreads();
   }
+}
+
+// The shared expert as one more expert of the table and one more pair of every row: one grouped GEMM does both.
+__global__ void a16_layer_prep_kernel(const uint8_t* const* __restrict__ tab, int E, const uint8_t* shared_rec, const int32_t* __restrict__ ids, int M, int K,
+                                      const uint8_t** __restrict__ tab2, int32_t* __restrict__ ids2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i <= E) tab2[i] = i < E ? tab[i] : shared_rec;
+  if (i < M * (K + 1)) { const int m = i / (K + 1), k = i - m * (K + 1); ids2[i] = k < K ? ids[m * K + k] : E; }
 }
 
 }  // namespace hb
@@ -617,9 +626,10 @@ A16Kernel a16_kernel(int bn) {
 // bf16 activations on the tensor cores: plan (tiles of ≤ 256 pairs) → slot-ordered copy of the rows → gate/up GEMM → down GEMM → sums.
 // The copy of the rows lives in the buffer of the per-pair down rows: the gate/up GEMM has read it before the down GEMM writes there.
 int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids, const float* w, int M, int K, const __nv_bfloat16* x, int H, int I, float limit,
-               float* out, const PfWs& W, int S, cudaStream_t st, const hb_pf_combine* cmb) {
+               float* out, const PfWs& W, int S, cudaStream_t st, const hb_pf_combine* cmb, bool shared_pair = false) {
   hb_rec_layout L;
   hb_rec_layout_make(H, I, &L);
+  const int Kr = shared_pair ? K - 1 : K;                      // routed pairs of a row: what w holds
   int r = hbk_moe_dtc_maps(ctx, lt, E, nullptr, H, I, st);
   if (r) return r;
   const size_t Pcap = (size_t)S * K;
@@ -644,7 +654,9 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
     const int n = M - s0 < S ? M - s0 : S, P = n * K;
     // the tile size by the pairs an expert gets on average: runs a standard deviation or two above it still fit one tile, and an
     // expert's weights are dequantised once per tile (39 pairs on average: 64 beats 128 beats 256; figures in pf_a16.cuh)
-    const A16Kernel gk = a16_kernel((long long)P <= 44ll * E ? 64 : (long long)P <= 100ll * E ? 128 : 256);
+    const long long routed = (long long)n * Kr;
+    const int experts = shared_pair ? E - 1 : E;
+    const A16Kernel gk = a16_kernel(routed <= 44ll * experts ? 64 : routed <= 100ll * experts ? 128 : 256);
     PlanArgs pl{ids + (size_t)s0 * K, P, E, lt, gk.bn, 1, W.hist, W.perm, W.pos_of, W.tiles, W.n_tiles, W.n_slots,
                 reinterpret_cast<unsigned int*>(ctx->dev_err) + kErrPlanMeet, ctx->dev_err};
     int plan_ctas = (P + 2047) / 2048;
@@ -662,9 +674,9 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
     common(1, &d);
     d.off_w = (uint32_t)L.w2; d.off_s0 = (uint32_t)L.s2; d.off_s1 = (uint32_t)L.s2; d.row2 = 64; d.out = W.part;
     if ((r = hb_launch(ctx, "a16_gemm_down", false, gk.fn, dim3(grid), dim3(A16_THREADS), gk.smem, st, d, tm_y))) return r;
-    const __nv_bfloat16* sh = cmb ? reinterpret_cast<const __nv_bfloat16*>(cmb->shared) + (size_t)s0 * H : nullptr;
+    const __nv_bfloat16* sh = cmb && cmb->shared ? reinterpret_cast<const __nv_bfloat16*>(cmb->shared) + (size_t)s0 * H : nullptr;
     if ((r = hb_launch(ctx, "pf_sum_pairs", false, pf_sum_pairs_kernel, dim3((unsigned)((n + SUM_ROWS - 1) / SUM_ROWS < ctx->sm_count * 8 ? (n + SUM_ROWS - 1) / SUM_ROWS : ctx->sm_count * 8)), dim3(256), 0, st,
-                       (const __nv_bfloat16*)W.part, (const int*)W.pos_of, w + (size_t)s0 * K, n, K, H, cmb ? (float*)nullptr : out + (size_t)s0 * H, sh,
+                       (const __nv_bfloat16*)W.part, (const int*)W.pos_of, w + (size_t)s0 * Kr, n, Kr, K, H, cmb ? (float*)nullptr : out + (size_t)s0 * H, sh,
                        cmb && cmb->lg ? cmb->lg + (size_t)s0 * cmb->ld : (const float*)nullptr, cmb ? cmb->ld : 0, cmb ? cmb->col : 0,
                        cmb ? reinterpret_cast<__nv_bfloat16*>(cmb->out) + (size_t)s0 * H : (__nv_bfloat16*)nullptr)))
       return r;
@@ -672,6 +684,31 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
   return HB_OK;
 }
 }  // namespace
+
+// The whole bf16-activation layer behind the router: routed and shared expert in one grouped GEMM (the shared expert apart took a plan, a
+// copy of the rows, two GEMM launches, a sum and a conversion of its own: 105 of 712 us at 1999 rows).
+size_t hbk_moe_layer_a16_ws_bytes(int M, int K, int E, int H, int I) {
+  return hb_align256((size_t)(E + 1) * 8) + hb_align256((size_t)M * (K + 1) * 4) + hb_moe_prefill_ws_bytes(M, K + 1, E + 1, H, I);
+}
+bool hbk_moe_layer_a16_takes(const hb_ctx* ctx, int M, int K, int E, int H, int I) {
+  return (ctx->flags & HB_FLAG_PREFILL_A16) && !(ctx->flags & HB_FLAG_PREFILL_A16_ROWS) && M > 64 && hb_moe_prefill_supported(H, I) && hbk_moe_dtc_supported(H, I) &&
+         E + 1 <= 1024 && K + 1 <= 32 && (long long)M * (K + 1) < (1ll << 30);
+}
+int hbk_moe_layer_a16(hb_ctx* ctx, const uint8_t* const* lt, int E, const uint8_t* shared_rec, const int32_t* ids, const float* w, int M, int K, const void* x, int H,
+                      int I, float limit, const float* lg, int ld, int col, void* out, void* ws, cudaStream_t st) {
+  HB_REQUIRE(ctx, hb_aligned(x, 16) && hb_aligned(out, 16), HB_ERR_INVALID, "moe_layer: x and the output must be 16-byte aligned");
+  char* p = static_cast<char*>(ws);
+  const uint8_t** tab2 = reinterpret_cast<const uint8_t**>(p); p += hb_align256((size_t)(E + 1) * 8);
+  int32_t* ids2 = reinterpret_cast<int32_t*>(p); p += hb_align256((size_t)M * (K + 1) * 4);
+  PfWs W;
+  pf_carve(p, M, K + 1, E + 1, H, I, &W);
+  const int n = M * (K + 1) > E + 1 ? M * (K + 1) : E + 1;
+  int r = hb_launch(ctx, "a16_layer_prep", false, a16_layer_prep_kernel, dim3((n + 255) / 256), dim3(256), 0, st, lt, E, shared_rec, ids, M, K, tab2, ids2);
+  if (r) return r;
+  hb_pf_combine cmb = {};
+  cmb.lg = lg; cmb.ld = ld; cmb.col = col; cmb.out = out;
+  return pf_a16_run(ctx, tab2, E + 1, ids2, w, M, K + 1, reinterpret_cast<const __nv_bfloat16*>(x), H, I, limit, nullptr, W, M, st, &cmb, true);
+}
 
 #ifdef HB_A16_TRACE
 extern "C" __attribute__((visibility("default"))) int hb_a16_trace_read(long long* out, int n) {
@@ -773,7 +810,7 @@ int hb_moe_prefill(hb_ctx* ctx, const uint8_t* const* rec_tab, int li, int E, co
     if ((r = pf_launch<PF_DOWN>(ctx, "pf_gemm_down", a, tm_y, tm_y, st))) return r;
     const __nv_bfloat16* sh = cmb ? reinterpret_cast<const __nv_bfloat16*>(cmb->shared) + (size_t)s0 * H : nullptr;
     if ((r = hb_launch(ctx, "pf_sum_pairs", false, pf_sum_pairs_kernel, dim3((unsigned)((n + SUM_ROWS - 1) / SUM_ROWS < ctx->sm_count * 8 ? (n + SUM_ROWS - 1) / SUM_ROWS : ctx->sm_count * 8)), dim3(256), 0, st,
-                       (const __nv_bfloat16*)W.part, (const int*)W.pos_of, w + (size_t)s0 * K, n, K, H, cmb ? (float*)nullptr : out + (size_t)s0 * H, sh,
+                       (const __nv_bfloat16*)W.part, (const int*)W.pos_of, w + (size_t)s0 * K, n, K, K, H, cmb ? (float*)nullptr : out + (size_t)s0 * H, sh,
                        cmb && cmb->lg ? cmb->lg + (size_t)s0 * cmb->ld : (const float*)nullptr, cmb ? cmb->ld : 0, cmb ? cmb->col : 0,
                        cmb ? reinterpret_cast<__nv_bfloat16*>(cmb->out) + (size_t)s0 * H : (__nv_bfloat16*)nullptr)))
       return r;

@@ -32,12 +32,14 @@ namespace hb {
 // operand, without touching shared memory (writing them to it and reading them back was what bounded small tiles: 1050 of 1600 clocks a
 // step with the MMAs waiting on it), and with ≤ 64 pairs the sums of two items, so the MMAs need not wait for the epilogue.  Measured for
 // 1999 rows of 512 experts (hidden 2048, intermediate 512, top-10: 39 pairs an expert), tiles of ≤ 256 in shared memory → ≤ 64 in tensor
-// memory, with the issuing threads elected: gate/up 440 → 375 µs, down 260 → 205 µs (routed part).
+// memory, the issuing threads elected, two steps a hand-over: gate/up 440 → 240 µs, down 260 → 145 µs.  What bounds it now is the
+// dequantisation (640 of 1030 clocks a step of 64 k values; the MMAs are busy for half of it).
 template <int BN_>
 struct A16Cfg {
   static constexpr int BN = BN_;                                     // pairs of a tile, at most
   static constexpr bool AT = BN <= 128;                              // the dequantised weights sit in tensor memory (else: swizzled tiles in shared memory)
-  static constexpr int STA = AT ? 4 : 2;                             // operand rings: dequantised weight tiles, activation tiles
+  static constexpr int KA = AT ? 2 : 1;                              // steps of 64 k values a weight stage holds: the hand-over of a stage costs as much as its values
+  static constexpr int STA = 2;                                      // operand rings: dequantised weight stages, activation tiles
   static constexpr int STB = BN <= 64 ? 8 : BN <= 128 ? 5 : 3;
   static constexpr int RAWS = AT ? 4 : 2;                            // raw code slots (256 k values each)
   static constexpr int NACC = BN <= 64 ? 2 : 1;                      // accumulator buffers of 2·BN columns
@@ -47,7 +49,7 @@ struct A16Cfg {
   static constexpr int RAW = 2 * A1;                                 // raw codes of both A tiles: 128 rows × 128 bytes each (256 k values per row)
   static constexpr int ACOL = NACC * 2 * BN;                         // tensor memory: accumulators, then stages of two A tiles of 32 columns (bf16 pairs)
   static constexpr int SMEM = 1024 + STA * A + STB * B + RAWS * RAW + 1024;
-  static_assert(SMEM <= 227 * 1024 && ACOL + (AT ? STA * 64 : 0) <= 512, "shared memory, tensor memory");
+  static_assert(SMEM <= 227 * 1024 && ACOL + (AT ? STA * KA * 64 : 0) <= 512, "shared memory, tensor memory");
 };
 constexpr int A16_BN_MAX = 256, A16_BN_MIN = 64;
 constexpr int A16_THREADS = 28 * 32;            // warps 0-3 and 4-7 epilogues of the two A tiles, 8 and 27 their MMAs, 9 raw codes, 10-17 and 18-25 dequantisation, 26 activations
@@ -255,6 +257,7 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
     }
     const int sbytes = a.K >> 4;                               // scale bytes per matrix row
     uint32_t rit = 0, kit = 0;
+    [[maybe_unused]] int pend = -1;                            // weight stage that is stored but not announced yet
     bool ok = true;
     [[maybe_unused]] long long tw = 0, tc = 0, t0 = clock64(), tl0 = 0;
     for (int item = blockIdx.x; item < n_items_all && ok; item += gridDim.x) {
@@ -272,41 +275,65 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
         if (!ok) break;
         const uint8_t* rawrow = smR + sl * C::RAW + u * C::A1 + rr * 128;
         const uint32_t scw[4] = {sc.x, sc.y, sc.z, sc.w};
-#pragma unroll
-        for (int kq = 0; kq < 4; ++kq, ++kit) {
-#ifdef HB_A16_TRACE
-          tl0 = clock64();
-#endif
-          const uint4 cw = *reinterpret_cast<const uint4*>(rawrow + (((kq * 2 + h) ^ (rr & 7)) << 4));     // 32 codes
+        auto dequant = [&](int kq, uint4& o0, uint4& o1, uint4& o2, uint4& o3) {                             // 32 codes of this thread's row
+          const uint4 cw = *reinterpret_cast<const uint4*>(rawrow + (((kq * 2 + h) ^ (rr & 7)) << 4));
           const uint32_t s2 = (scw[kq] >> (16 * h)) & 0xffffu;                                              // the two block scales
           const uint32_t sh = f16x2_to_bf16x2(cvt_e4m3x2_f16x2(s2));
           const uint32_t slo = __byte_perm(sh, sh, 0x1010), shi = __byte_perm(sh, sh, 0x3232);             // (s0, s0), (s1, s1) as bf16
-          const uint4 o0 = a16_dequant8(cw.x, slo), o1 = a16_dequant8(cw.y, slo), o2 = a16_dequant8(cw.z, shi), o3 = a16_dequant8(cw.w, shi);
+          o0 = a16_dequant8(cw.x, slo); o1 = a16_dequant8(cw.y, slo); o2 = a16_dequant8(cw.z, shi); o3 = a16_dequant8(cw.w, shi);
+        };
+        if constexpr (C::AT) {
+          // two steps a stage; the stage before is announced after this one's first values are worked out (its stores have landed by then)
+#pragma unroll
+          for (int kq = 0; kq < 4; ++kq) {
 #ifdef HB_A16_TRACE
-          if (o0.x == 0x12345u && o3.w == 0x54321u) tc += 1;            // keeps the values' computation in front of the clock read
-          tc += clock64() - tl0;
+            tl0 = clock64();
 #endif
-          // one lane waits for the slot and one lane announces the warp's rows
-          const uint32_t sa = kit % C::STA;
-          if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&emptyA[sa], ((kit / C::STA) & 1u) ^ 1u, a.err, 0x8u));
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
-          if constexpr (C::AT) {
-            tc_fence_after();
+            uint4 o0, o1, o2, o3;
+            dequant(kq, o0, o1, o2, o3);
+#ifdef HB_A16_TRACE
+            if (o0.x == 0x12345u && o3.w == 0x54321u) tc += 1;
+            tc += clock64() - tl0;
+#endif
+            const uint32_t sa = kit % C::STA;
+            if (kq % C::KA == 0) {
+              if (pend >= 0) { tc_wait_st(); tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(&fullA[pend]); }
+              A16_TIMED(tw, ok = mbar_wait(&emptyA[sa], ((kit / C::STA) & 1u) ^ 1u, a.err, 0x8u));
+              ok = __all_sync(0xffffffffu, ok);
+              pend = -1;
+              if (!ok) break;
+              tc_fence_after();
+            }
             const uint32_t w16[16] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w, o2.x, o2.y, o2.z, o2.w, o3.x, o3.y, o3.z, o3.w};
-            tc_st16(acol + sa * 64, w16);
-            tc_wait_st();
-            tc_fence_before();
-          } else {
+            tc_st16(acol + (sa * C::KA + kq % C::KA) * 64, w16);
+            if (kq % C::KA == C::KA - 1) { pend = (int)sa; ++kit; }
+          }
+        } else {
+#pragma unroll
+          for (int kq = 0; kq < 4; ++kq, ++kit) {
+#ifdef HB_A16_TRACE
+            tl0 = clock64();
+#endif
+            uint4 o0, o1, o2, o3;
+            dequant(kq, o0, o1, o2, o3);
+#ifdef HB_A16_TRACE
+            if (o0.x == 0x12345u && o3.w == 0x54321u) tc += 1;            // keeps the values' computation in front of the clock read
+            tc += clock64() - tl0;
+#endif
+            // one lane waits for the slot and one lane announces the warp's rows
+            const uint32_t sa = kit % C::STA;
+            if (lane == 0) A16_TIMED(tw, ok = mbar_wait(&emptyA[sa], ((kit / C::STA) & 1u) ^ 1u, a.err, 0x8u));
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
             uint8_t* arow = smA + sa * C::A + u * C::A1 + r * 128;
             *reinterpret_cast<uint4*>(arow + (((h * 4 + 0) ^ (r & 7)) << 4)) = o0;
             *reinterpret_cast<uint4*>(arow + (((h * 4 + 1) ^ (r & 7)) << 4)) = o1;
             *reinterpret_cast<uint4*>(arow + (((h * 4 + 2) ^ (r & 7)) << 4)) = o2;
             *reinterpret_cast<uint4*>(arow + (((h * 4 + 3) ^ (r & 7)) << 4)) = o3;
             fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&fullA[sa]);
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&fullA[sa]);
         }
         if (!ok) break;
         __syncwarp();
@@ -314,6 +341,7 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
         sc = sc_next;
       }
     }
+    if (C::AT && pend >= 0) { tc_wait_st(); tc_fence_before(); __syncwarp(); if (lane == 0) mbar_arrive(&fullA[pend]); }
     if (dt == 0) { A16_PUT(2, tw); A16_PUT(3, clock64() - t0); A16_PUT(4, tc); }
   } else if (warp == A16_W_MMA || warp == A16_W_MMA1) {
     // ------------------------------------------------------------------------------------------------ MMA issue: one thread per A tile (one thread for both spent a
@@ -338,20 +366,23 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
         for (int kb = 0; kb < nk; ++kb) {
           A16_TIMED(twb, ok = mbar_wait(&fullB[sb], pb, a.err, 0x40u));
           if (!ok) break;
-          A16_TIMED(twa, ok = mbar_wait(&fullA[sa], pa, a.err, 0x20u));
+          const int ka = kb % C::KA;                                // step within the weight stage (nk is a multiple of four)
+          if (ka == 0) A16_TIMED(twa, ok = mbar_wait(&fullA[sa], pa, a.err, 0x20u));
           if (!ok) break;
           tc_fence_after();
           const uint64_t ad = ad0 + sa * (uint32_t)(C::A >> 4), bd = bd0 + sb * (uint32_t)(C::B >> 4);
-          const uint32_t at = tmem + C::ACOL + sa * 64 + uu * 32;
+          const uint32_t at = tmem + C::ACOL + (sa * C::KA + ka) * 64 + uu * 32;
 #pragma unroll
           for (uint32_t j = 0; j < 4; ++j) {
             if constexpr (C::AT) tc_mma_f16_at(acc, at + 8 * j, bd + 2 * j, idesc, j ? 1u : more);
             else tc_mma_f16(acc, ad + 2 * j, bd + 2 * j, idesc, j ? 1u : more);
           }
           more = 1u;
-          tc_commit(&emptyA[sa]);
           tc_commit(&emptyB[sb]);
-          if (++sa == C::STA) { sa = 0; pa ^= 1u; }
+          if (ka == C::KA - 1) {
+            tc_commit(&emptyA[sa]);
+            if (++sa == C::STA) { sa = 0; pa ^= 1u; }
+          }
           if (++sb == C::STB) { sb = 0; pb ^= 1u; }
 #ifdef HB_A16_TRACE
           ++kit;

@@ -349,3 +349,24 @@ def test_moe_prefill_degenerate_inputs(E, oracle):
     assert _lib.load().hb_moe_prefill(ctx.handle, tab.data_ptr(), 0, E_, ids.data_ptr(), w.data_ptr(), 0, K, x.data_ptr(), H, I, 0.0, out.data_ptr(),
                                       ws.data_ptr(), 8, None, None) == 0
 
+
+
+@pytest.mark.parametrize("M,E_,K", [(65, 8, 2), (129, 4, 2), (333, 8, 3), (700, 4, 2), (66, 1024, 2)])
+def test_moe_layer_shared_expert_in_the_grouped_gemm(E, oracle, M, E_, K):
+    """hb_moe_layer with bf16 activations runs the shared expert as one more expert of the grouped GEMM: the same bits as the shared expert
+    apart (a one-expert routing of weight 1) followed by the routed experts with the fused combine, at every tile size of the GEMM, and
+    where the table has no room for one more expert (1024)."""
+    H, I = 512, 256
+    dev = torch.device("cuda")
+    keep = upload(random_records(oracle, H, I, 9, M + E_), dev)
+    tab = E.rec_table([keep[e % 8] for e in range(E_)])
+    g = torch.Generator(device="cpu").manual_seed(M)
+    x = torch.randn((M, H), generator=g).to(torch.bfloat16).to(dev)
+    logits = torch.randn((M, E_ + 1), generator=g).to(dev)
+    ctx = E.Context(flags=E.HB_FLAG_PREFILL_A16)
+    ids, w, out = E.moe_layer(logits, x, tab, 0, E_, K, H, I, shared_rec=keep[8], gate_col=E_, ctx=ctx)
+    one = torch.zeros((M, 1), dtype=torch.int32, device=dev)
+    sh = E.fn_moe_prefill(E.rec_table([keep[8]]), 0, 1, one, torch.ones((M, 1), device=dev), x, H, I, ctx=ctx).to(torch.bfloat16)
+    ref = E.fn_moe_prefill(tab, 0, E_, ids, w, x, H, I, shared=sh, lg=logits, col=E_, ctx=ctx)
+    assert torch.equal(out.view(torch.int16), ref.view(torch.int16))
+    ctx.check_device()
