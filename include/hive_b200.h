@@ -51,7 +51,7 @@ typedef struct hb_config {
 #define HB_FLAG_DECODE_TC 16      /* same as HB_FLAG_DECODE_TC_GU (kept for callers that set it) */
 #define HB_FLAG_DECODE_TC_GU 64   /* decode, routed operators: the gate/up pass runs on the tensor-memory kernel (exact digit planes of the activations,
                                      block-scaled FP4 MMAs) at every size, grouping and down pass on the streaming kernels.  With neither flag the
-                                     library picks by the number of pairs of the call (40 or more: tensor memory); both engines meet the same
+                                     library picks by the size of the call (pairs · H · I of 16 Mi or more: tensor memory); both engines meet the same
                                      tolerance, and a row's bits do not depend on its batch as long as the engine does not change — pin one
                                      with a flag where that matters */
 #define HB_FLAG_DECODE_TC_DOWN 128 /* decode, routed operators on one GPU: where the gate/up pass runs on the tensor-memory kernel, the down pass does too
@@ -255,7 +255,7 @@ HB_API int hb_moe_layer_decode(hb_ctx* ctx, const float* logits, int ld, int M, 
 HB_API size_t hb_dense_gemv_ws_bytes(int fmt, int N, int K, int n_mats /* 1 = gemv, 2 = gemv_gu */);
 /* hive::q27::k::gemv — engine/include/hive/q27/q27_kernels.h:48-50, engine/src/q27/q27_kernels.cu:2423-2449:
  * y[m,n] = Σ_k x[m,k]·W[n,k], fp32 accumulation, written as bf16 (yb) or fp32 (yf): exactly one non-NULL.  x bf16 [M,K] (row
- * stride ldx), M ≤ 16 (the reference takes ≤ 8; rows are processed 8 at a time with batch-independent arithmetic), K % 256 == 0. */
+ * stride ldx), M ≤ 16 (the reference takes ≤ 8; a row's result does not depend on the rows beside it), K % 256 == 0. */
 HB_API int hb_dense_gemv(hb_ctx* ctx, const hb_qmat* W, const void* x_bf16, int ldx, int M, void* yb_bf16, float* yf, int ldy, void* ws,
                          void* stream);
 /* hive::q27::k::gemv_gu — engine/include/hive/q27/q27_kernels.h:62-64, engine/src/q27/q27_kernels.cu:258-289:
