@@ -935,7 +935,7 @@ def dense_measure(args, torch, E, ctx, dev, Ms=(1, 8)):
     return {"metric": "dense_ffn_layer_GBps", "value": head["achieved_GBps"], "unit": "GB/s", "n_gpus": 1, "data": "synthetic",
             "config": {"workload": "dense 27B-style MLP decode: hidden 5120, FFN 17408, gate/up + down GEMV, M in %s" % (list(Ms),),
                        "l2": "12 layers' matrices cycled (1.2-1.8 GB, larger than L2)"},
-            "roofline": {"bound": "hbm", "kernel": "dense_stream_kernel", "achieved": head["achieved_GBps"], "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "hbm", "kernel": "dense_gemv_kernel", "achieved": head["achieved_GBps"], "peak": peak, "unit": "GB/s",
                          "frac": head["frac_of_measured_hbm"], "traffic": None},
             "per_case": res}
 
