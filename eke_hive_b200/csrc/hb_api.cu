@@ -312,7 +312,10 @@ size_t layer_carve(void* ws, int M, int K, int E, int H, int I, LayerWs* w) {
   LayerWs t;
   const bool pf = M > kDecodeRows && hb_moe_prefill_supported(H, I) > 0;
   const int rows = M < kDecodeRows ? M : kDecodeRows;
-  t.op = take(pf ? hb_moe_prefill_ws_bytes(M, K, E, H, I) : hb_moe_decode_ws_bytes(rows * (K + 1), H, I));
+  // the size does not know the context's flags: more than 64 rows run either as one grouped GEMM or as decode calls of 64 rows, whose
+  // scratch is the larger one up to some 130 rows
+  const size_t dec = hb_moe_decode_ws_bytes(rows * (K + 1), H, I), gemm = pf ? hb_moe_prefill_ws_bytes(M, K, E, H, I) : 0;
+  t.op = take(dec > gemm ? dec : gemm);
   t.tab1 = (const uint8_t**)take(256); t.ids1 = (int32_t*)take(pf ? (size_t)M * 4 : 0); t.w1 = (float*)take(pf ? (size_t)M * 4 : 0);
   t.sh32 = (float*)take(pf ? (size_t)M * H * 4 : 0); t.sh16 = take(pf ? (size_t)M * H * 2 : 0);
   if (w) *w = t;

@@ -77,6 +77,17 @@ def test_workspace_and_support_queries(lib):
     assert a % 256 == 0 and a >= 176 * (2048 + 512) * 2 and a < b < 2 * a + 4096
 
 
+def test_layer_workspace_holds_the_decode_calls(lib):
+    """hb_moe_layer runs more than 64 rows as decode calls of 64 rows on a context that asked for no grouped GEMM: its workspace holds such a
+    call's scratch (shared expert's pairs included) at every row count, and the grouped GEMM's."""
+    L = lib.load()
+    for H, I, E, K in ((2048, 512, 512, 10), (4096, 1536, 160, 8), (7168, 2048, 256, 8), (256, 256, 4, 1), (512, 256, 1024, 16)):
+        for M in (1, 63, 64, 65, 66, 100, 127, 128, 129, 190, 191, 300, 5000):
+            ws = L.hb_moe_layer_ws_bytes(M, K, E, H, I)
+            assert ws >= L.hb_moe_decode_ws_bytes(min(M, 64) * (K + 1), H, I), (H, I, E, K, M)
+            assert M <= 64 or ws >= L.hb_moe_prefill_ws_bytes(M, K, E, H, I), (H, I, E, K, M)
+
+
 def test_status_strings_and_null_context(lib):
     L = lib.load()
     assert L.hb_status_string(0) == b"ok" and b"unsupported" in L.hb_status_string(-2)
