@@ -759,10 +759,14 @@ int hb_moe_prefill(hb_ctx* ctx, const uint8_t* const* rec_tab, int li, int E, co
     // this operator's workspace)
     int rows = HB_MAX_PAIRS / K < S ? HB_MAX_PAIRS / K : S;
     HB_REQUIRE(ctx, rows >= 1 && hb_moe_decode_supported(H, I) > 0, HB_ERR_UNSUPPORTED, "moe_prefill (bf16 activations): K=%d H=%d I=%d", K, H, I);
-    while (rows > 1 && hbk_moe_decode_ws_bytes(rows * K, H, I) > hb_moe_prefill_ws_bytes(S, K, E, H, I)) rows /= 2;
+    const size_t have = hb_moe_prefill_ws_bytes(S, K, E, H, I);
+    while (rows > 1 && hbk_moe_decode_ws_bytes(rows * K, H, I) > have) rows /= 2;
+    // one row at a time and few experts: this operator's workspace holds the streaming kernels' scratch, not the digit planes
+    const bool stream_only = hbk_moe_decode_ws_bytes(rows * K, H, I) > have;
     for (int m0 = 0; m0 < M; m0 += rows) {
       const int n = M - m0 < rows ? M - m0 : rows;
       hbk_pair_src src; src.ids = ids + (size_t)m0 * K; src.w = w + (size_t)m0 * K; src.M = n; src.K = K; src.tab = rec_tab; src.li = li; src.E = E;
+      src.ws_stream_only = stream_only;
       src.pairs_hint = M * K;                                               // every sub-chunk runs on the engine the whole call would get
       hbk_reduce red;
       if (cmb) {
