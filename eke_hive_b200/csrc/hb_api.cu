@@ -49,7 +49,6 @@ int hb_create(const hb_config* cfg, hb_ctx** out) {
 void hb_destroy(hb_ctx* ctx) {
   if (!ctx) return;
   if (ctx->dev_err) cudaFree(ctx->dev_err);
-  if (ctx->dtc_maps) cudaFree(ctx->dtc_maps);
   if (ctx->prof_ev) {
     for (int i = 0; i < 2 * hb_ctx::kProfMax; ++i) cudaEventDestroy(ctx->prof_ev[i]);
     delete[] ctx->prof_ev;
@@ -129,7 +128,7 @@ int hb_check_device(hb_ctx* ctx, void* stream) {
   if (v & 0x80000000u)
     return hb_fail(ctx, HB_ERR_DEVICE_FLAG, "device error word 0x%x: range check 0x%x failed with value %d (debug build)", v, site[0], (int)site[1]);
   return hb_fail(ctx, HB_ERR_DEVICE_FLAG, "device error word 0x%x (bits 0x1-0x80: a pipeline wait inside a decode or prefill kernel; 0x400-0x2000: the decode layer kernel's tables and grid barrier; "
-                 "0x40000: rows of another rank did not arrive; 0x80000: partial sums of another rank did not arrive; 0x400000: an expert record outside the tensor maps' range)", v);
+                 "0x40000: rows of another rank did not arrive; 0x80000: partial sums of another rank did not arrive; 0x400000: an expert record that is not 16-byte aligned)", v);
 }
 
 int hb_rec_layout_make(int H, int I, hb_rec_layout* L) {

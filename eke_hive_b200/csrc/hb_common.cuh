@@ -26,9 +26,9 @@ struct hb_ctx {
   int smem_optin = 0;            // cudaDevAttrMaxSharedMemoryPerBlockOptin
   uint32_t* dev_err = nullptr;   // device error word: 0 = fine; kernels OR a site code into it when a bounded wait gives up
   unsigned long long launches = 0;
-  // tensor maps of the decode layer kernel (k_moe_dtc.cu): device array + the shape they were made for
-  void* dtc_maps = nullptr;
-  int dtc_H = 0, dtc_I = 0;
+  // encoded weight maps without a base, by row pitch (wmap.cuh): functions of the pitch alone, copied into each launch that stamps maps
+  struct WmTemplate { int pitch = 0; alignas(64) unsigned char map[128]; };
+  WmTemplate wm_tpl[4]; int wm_next = 0;
   // streaming down kernels (one per split-K width): whether the planned number of CTAs per SM is really resident, i.e. whether the
   // CTAs may meet inside the kernel (k_moe_decode.cu)
   const void* down_fn[8] = {nullptr}; bool down_meet[8] = {false};

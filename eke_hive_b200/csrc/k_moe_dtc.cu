@@ -18,13 +18,13 @@
 //
 // The kernel: persistent CTAs, one per SM.  Work item = (group, 64 rows of I: 64 gate rows + 64 up rows form one 128-row A tile),
 // dealt round-robin; a CTA's list is closed-form and built once into shared memory.  Per CTA: one thread streams weight boxes
-// (128 bytes × 64 rows, 128-byte swizzle) by TMA through a tensor map anchored below the records; one thread copies the digit
+// (128 bytes × 64 rows, 128-byte swizzle) by TMA through the call's own weight maps (wmap.cuh); one thread copies the digit
 // planes (pre-swizzled 1 KB atoms, plain bulk copies); four warps fetch the e4m3 scale rows ahead with cp.async and store them into
 // tensor memory with tcgen05.st; one thread issues the MMAs (128 × 16 × 64) into two accumulator buffers; two sets of four warps
 // run the epilogue (Horner, global scales, SwiGLU, y).  Every wait is bounded and reports through the context's error word.
 #include "moe_stream.cuh"
 #include "ep.cuh"
-#include "tc_common.cuh"
+#include "wmap.cuh"
 
 namespace hb {
 
@@ -48,24 +48,17 @@ constexpr int DT_W_MMA = 8, DT_W_TMA = 9, DT_W_DIG = 10, DT_W_SC0 = 12;
 constexpr int DT_TMEM_COLS = 512;              // accumulators 2 × 64 columns, then 16 columns of weight scales per stage, then 16 columns of 1.0
 constexpr int DT_SFA_COL0 = 128;
 constexpr int DT_SFB1_COL = DT_SFA_COL0 + DT_ST * 16;   // the digit planes' block scales: 1.0 for every plane, written once
-constexpr int DT_VMAX = 32;                    // tensor-map variants (see DtcMeta)
 constexpr int DT_GU_ROWS = 64;                 // rows of I per item
 static_assert(DT_STAGE % 1024 == 0, "stage buffers keep the swizzle atom's alignment");
 static_assert(DT_SFB1_COL + 16 <= DT_TMEM_COLS, "tensor memory");
 static_assert(DT_SMEM <= 227 * 1024, "shared memory");
 static_assert(DT_ROWS <= kGroupRows, "groups of the grouping kernel");
 
-// A tensor map for the weight boxes cannot be made per record ahead of time (the table may change between calls) and records sit
-// at arbitrary 4096-aligned addresses.  One map covers them all: a 2-D byte matrix [2^31 rows][pitch] whose base lies 2^30 rows
-// below the lowest record seen when the map was made.  A matrix whose distance from that base is not a multiple of the pitch uses
-// variant v of the map, shifted by v·gcd(pitch, 4096) bytes (pitch / gcd variants cover every residue).
-struct DtcMeta { unsigned long long anchor; };
-
 struct DtcWs {
   uint8_t* xdig;        // [rows][K/256][8 planes][128 bytes], swizzled
   float* xs;            // [rows] unit of a row's digits (a power of two)
 };
-struct DtcWs2 { DtcWs x, y; };   // planes of the activation rows (K = H) and of the y rows (K = I)
+struct DtcWs2 { DtcWs x, y; uint8_t* maps; };   // planes of the activation rows (K = H) and of the y rows (K = I); the weight maps of both passes
 
 // Division of a 32-bit unsigned number by a divisor fixed for the whole launch: multiply-high and shift (exact for n < 2^31).
 struct DtDiv {
@@ -86,8 +79,7 @@ struct DtcArgs {
   DtDiv dIT, dG;                                          // dividers by the items per group and by the grid size
   uint32_t off_w, off_s0, off_s1, off_g;                  // record offsets: the matrix of the tile's first half, the scales of both halves, the global scales
   int row2, trows;                                        // matrix rows from the first 64-row box of an item to the second; matrix rows an item advances per half
-  const CUtensorMap* maps; const DtcMeta* meta;           // maps[variant]
-  int pitch, gstep, pshift;                               // pshift: log2(pitch) when the pitch divides 4096, else -1
+  WmArgs wm;                                              // the weight maps of this pass
   DtcWs dw;                                               // the digit planes of the B operand's rows
   __nv_bfloat16* out;                                     // bf16 [position, out_ld]
   unsigned int* fin; ReduceArgs red; int red_on;          // down: the sums over each row's pairs after the CTAs have met
@@ -199,10 +191,7 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
     mbar_fence_init();
   }
   if (warp == DT_W_MMA) { tmem_alloc(tmem_slot, DT_TMEM_COLS); tmem_relinquish(); }
-  // the first variant of the tensor map (the only one when the pitch divides 4096) is made visible to the TMA thread before the
-  // wait: the maps were stamped by an earlier launch that has completed
-  if (warp == DT_W_TMA) tmap_acquire(a.maps);                                  // by every lane: whichever of them is elected below
-  griddep_wait();                                                               // the group list and the digit planes of the rows
+  griddep_wait();                                                               // the group list, the digit planes of the rows and the weight maps
   griddep_launch();
   const int nIT = (int)a.dIT.d, grid = (int)a.dG.d, c0 = (int)blockIdx.x;
   const int n_gu = a.hdr[0] * nIT;
@@ -228,26 +217,16 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
   if (warp == DT_W_TMA) {
     // ------------------------------------------------------------------------------------------------ weight boxes: one thread
     if (elect_one()) {
-      uint32_t it = 0, seen = 1u;                                                // variant 0: acquired in the prologue
+      uint32_t it = 0;
       bool ok = true;
       [[maybe_unused]] long long tw = 0, t_begin = clock64();
-      const unsigned long long anchor = a.meta->anchor;
+      WmReader wm;
+      wm.init(a.wm);
       for (int ii = 0; ii < n_items && ok; ++ii) {
         const DtEnt e = tbl[ii];
-        const unsigned long long addr = reinterpret_cast<unsigned long long>(e.rec) + a.off_w, delta = addr - anchor;
-        unsigned long long row;
-        int v = 0;
-        if (a.pshift >= 0) row = delta >> a.pshift;                               // the pitch divides 4096: every matrix is a whole number of rows above the anchor
-        else {
-          const unsigned long long rem = delta % (unsigned long long)a.pitch;
-          row = (delta - rem) / (unsigned long long)a.pitch;
-          v = (int)(rem / (unsigned long long)a.gstep);
-          if (rem % (unsigned long long)a.gstep || v >= DT_VMAX) { atomicOr(a.err, 0x400000u); break; }
-        }
-        if (addr < anchor || row + (1ull << 24) >= (1ull << 31)) { atomicOr(a.err, 0x400000u); break; }
-        const CUtensorMap* map = a.maps + v;
-        if (!((seen >> v) & 1u)) { tmap_acquire(map); seen |= 1u << v; }
-        const int r0 = (int)row + ent_t(e) * a.trows, r1 = r0 + a.row2;
+        WmBox box;
+        if (!wm.locate(e.rec + a.off_w, box, a.err)) break;
+        const int r0 = ent_t(e) * a.trows, r1 = r0 + a.row2;
         for (int kb = 0; kb < nkb; ++kb, ++it) {
           const uint32_t stage = it % DT_ST;
           DT_TIMED(tw, ok = mbar_wait(&empty[stage], ((it / DT_ST) & 1) ^ 1, a.err, 0x1u));
@@ -255,8 +234,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
           DT_STAMP(it, 0);
           const uint32_t sb = base + stage * DT_STAGE;
           mbar_expect_tx(&full[stage], DT_A);
-          tma_load_2d(sb, map, kb * 128, r0, &full[stage]);                       // 64 gate rows | rows 0-63 of the w2 tile
-          tma_load_2d(sb + DT_A / 2, map, kb * 128, r1, &full[stage]);            // 64 up rows | rows 64-127
+          wm.load(sb, box, kb * 128, r0, &full[stage]);                           // 64 gate rows | rows 0-63 of the w2 tile
+          wm.load(sb + DT_A / 2, box, kb * 128, r1, &full[stage]);                // 64 up rows | rows 64-127
           DT_STAMP(it, 1);
         }
       }
@@ -483,12 +462,18 @@ __global__ void __launch_bounds__(DT_THREADS, 1) moe_dtc_layer_kernel(const DtcA
 // wait_flags: the rows are pushed by other ranks (expert parallel) — every CTA waits, bounded, for the same flags the grouping kernel
 // waits for before it reads its row.
 // wait_first: the rows are the previous kernel's output (the y rows between the two passes): wait for it before reading.
-struct XdigArgs { const __nv_bfloat16* x; int x_ld, H; DtcWs dw; const uint32_t* wait_flags; int wait_n; const uint32_t* wait_step; uint32_t* err; int wait_first; };
-__global__ void __launch_bounds__(256) moe_xdig_kernel(const XdigArgs a) {
+// One CTA more than rows: the last one stamps the weight maps of both passes (the table is as final as the rows are).
+struct XdigArgs { const __nv_bfloat16* x; int x_ld, H, M; DtcWs dw; const uint32_t* wait_flags; int wait_n; const uint32_t* wait_step; uint32_t* err; int wait_first; };
+__global__ void __launch_bounds__(256) moe_xdig_kernel(const XdigArgs a, const __grid_constant__ WmStamp wm) {
   __shared__ int s_red[8];
   const int m = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   griddep_launch();
   if (a.wait_first) griddep_wait();
+  if (m == a.M) {
+    wm_stamp(wm);
+    if (!a.wait_first) griddep_wait();
+    return;
+  }
   if (a.wait_flags) {
     if ((int)threadIdx.x < a.wait_n && !*reinterpret_cast<volatile uint32_t*>(a.err)) ep_wait_flag(a.wait_flags + threadIdx.x, *a.wait_step + 1u, a.err, 0x40000u);
     __syncthreads();
@@ -515,49 +500,20 @@ __global__ void __launch_bounds__(256) moe_xdig_kernel(const XdigArgs a) {
   if (!a.wait_first) griddep_wait();
 }
 
-// Stamps the anchored base into the variants of the tensor map (one block; runs when the maps are first needed).
-struct DtcMapTpl { CUtensorMap t; };
-__global__ void moe_dtc_anchor_kernel(const __grid_constant__ DtcMapTpl tpl, const uint8_t* const* __restrict__ tab, int n_tab, const uint8_t* shared_rec,
-                                      int pitch, int gstep, CUtensorMap* __restrict__ maps, DtcMeta* __restrict__ meta) {
-  __shared__ unsigned long long s_min;
-  if (threadIdx.x == 0) s_min = shared_rec ? reinterpret_cast<unsigned long long>(shared_rec) : ~0ull;
-  __syncthreads();
-  unsigned long long mn = ~0ull;
-  for (int i = threadIdx.x; i < n_tab; i += blockDim.x) { const unsigned long long p = reinterpret_cast<unsigned long long>(tab[i]); if (p) mn = min(mn, p); }
-  atomicMin(&s_min, mn);
-  __syncthreads();
-  const unsigned long long lo = s_min == ~0ull ? (1ull << 40) : (s_min & ~4095ull);
-  for (int v = threadIdx.x; v < DT_VMAX; v += blockDim.x) {
-    if (v >= pitch / gstep) continue;
-    unsigned long long anchor = lo - ((unsigned long long)pitch << 30);
-    anchor &= ~4095ull;
-    if (v == 0) meta->anchor = anchor;
-    const uint4* src = reinterpret_cast<const uint4*>(&tpl.t);
-    uint4* dst = reinterpret_cast<uint4*>(maps + v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dst[j] = src[j];
-    const unsigned long long addr = anchor + (unsigned long long)v * gstep;
-    asm volatile("tensormap.replace.tile.global_address.global.b1024.b64 [%0], %1;" ::"l"(dst), "l"(addr) : "memory");
-    asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
-  }
-}
-
 }  // namespace hb
 
 using namespace hb;
 
 namespace {
-int gcd_int(int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; }
-
 size_t dtc_carve(void* ws, size_t off, int n, int H, int I, DtcWs2* w) {
   auto take = [&](size_t b) { void* r = ws ? static_cast<char*>(ws) + off : nullptr; off += al256(b); return r; };
   DtcWs2 t;
   t.x.xdig = (uint8_t*)take((size_t)n * 4 * H); t.x.xs = (float*)take((size_t)n * 4);
   t.y.xdig = (uint8_t*)take((size_t)n * 4 * I); t.y.xs = (float*)take((size_t)n * 4);
+  t.maps = (uint8_t*)take(wm_bytes(H) + wm_bytes(I));
   if (w) *w = t;
   return off;
 }
-constexpr size_t kMapSetBytes = (size_t)DT_VMAX * sizeof(CUtensorMap) + 256;   // the variants of one map and its DtcMeta
 int dtc_grid(const hb_ctx* ctx) {
   int grid = ctx->sm_count;
   if (ctx->max_ctas > 0 && grid > ctx->max_ctas) grid = ctx->max_ctas;
@@ -569,7 +525,7 @@ long long dtc_groups(int P, int E) { return P < E + 1 + P / DT_ROWS ? P : E + 1 
 bool hbk_moe_dtc_supported(int H, int I) {
   if (H <= 0 || I <= 0 || H % 256 || I % 256 || I / DT_GU_ROWS > 2047) return false;
   const int p0 = H / 2, p1 = I / 2;
-  return p0 / gcd_int(p0, 4096) <= DT_VMAX && p1 / gcd_int(p1, 4096) <= DT_VMAX && H / 128 <= 2047;
+  return p0 / wm_gcd4096(p0) <= kWmVariants && p1 / wm_gcd4096(p1) <= kWmVariants && H / 128 <= 2047;
 }
 
 // a CTA's list holds its share of the items
@@ -588,56 +544,40 @@ size_t hbk_moe_dtc_ws_extra(int n, int H, int I) { return hbk_moe_dtc_supported(
 
 int hbk_moe_dtc_setup(hb_ctx* ctx) {
   HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(moe_dtc_layer_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, DT_SMEM));
-  HB_CUDA(ctx, cudaMalloc(&ctx->dtc_maps, 2 * kMapSetBytes));
-  HB_CUDA(ctx, cudaMemset(ctx->dtc_maps, 0, 2 * kMapSetBytes));
   return HB_OK;
 }
 
-// the tensor maps of both passes (row pitch H/2 for gate and up, I/2 for down), anchored below the records of `tab`: made on first
-// use and whenever the shape changes
-static int dtc_maps_for(hb_ctx* ctx, const uint8_t* const* tab, int n_tab, const uint8_t* shared_rec, int H, int I, cudaStream_t st) {
-  if (ctx->dtc_H == H && ctx->dtc_I == I) return HB_OK;
+// the encoded map of a pitch (a byte matrix [2^31 rows][pitch], boxes of 128 bytes × 64 rows, 128-byte swizzle) with some base
+static int wm_template(hb_ctx* ctx, int pitch, const void* any, CUtensorMap* out) {
+  for (const auto& t : ctx->wm_tpl) if (t.pitch == pitch) { memcpy(out, t.map, sizeof *out); return HB_OK; }
   TcEncodeFn fn = tc_encode_fn();
   HB_REQUIRE(ctx, fn, HB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  for (int kind = 0; kind < 2; ++kind) {
-    DtcMapTpl tpl;
-    const int pitch = (kind ? I : H) / 2;
-    const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)1 << 31}, strides[1] = {(cuuint64_t)pitch};
-    const cuuint32_t box[2] = {128u, 64u}, estr[2] = {1, 1};
-    CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(static_cast<char*>(ctx->dtc_maps) + kind * kMapSetBytes);
-    const CUresult cr = fn(&tpl.t, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, maps, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    HB_REQUIRE(ctx, cr == CUDA_SUCCESS, HB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for pitch %d", (int)cr, pitch);
-    DtcMeta* meta = reinterpret_cast<DtcMeta*>(maps + DT_VMAX);
-    const int r = hb_launch(ctx, "moe_dtc_anchor", false, moe_dtc_anchor_kernel, dim3(1), dim3(256), 0, st, tpl, tab, n_tab, shared_rec, pitch,
-                            gcd_int(pitch, 4096), maps, meta);
-    if (r) return r;
-  }
-  ctx->dtc_H = H; ctx->dtc_I = I;
+  const cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)1 << 31}, strides[1] = {(cuuint64_t)pitch};
+  const cuuint32_t box[2] = {128u, 64u}, estr[2] = {1, 1};
+  const CUresult cr = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(any), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  HB_REQUIRE(ctx, cr == CUDA_SUCCESS, HB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for pitch %d", (int)cr, pitch);
+  auto& t = ctx->wm_tpl[ctx->wm_next++ % 4];
+  t.pitch = pitch;
+  memcpy(t.map, out, sizeof *out);
   return HB_OK;
 }
 
-// what both passes share: the list, the map set of the pass, the dividers
-static void dtc_args_common(hb_ctx* ctx, const DecodeWs& w, int kind, int K, int items_per_group, DtcArgs* a) {
-  a->hdr = w.hdr; a->groups = w.groups; a->down = kind; a->K = K; a->err = ctx->dev_err;
-  a->maps = reinterpret_cast<const CUtensorMap*>(static_cast<const char*>(ctx->dtc_maps) + kind * kMapSetBytes);
-  a->meta = reinterpret_cast<const DtcMeta*>(a->maps + DT_VMAX);
-  a->pitch = K / 2; a->gstep = gcd_int(K / 2, 4096);
-  a->pshift = -1;
-  for (int b = 7; b <= 12; ++b) if (a->pitch == (1 << b)) a->pshift = b;
-  a->dIT.set((uint32_t)items_per_group); a->dG.set((uint32_t)dtc_grid(ctx));
+int hbk_wm_stamp_args(hb_ctx* ctx, const uint8_t* const* tab, int n_tab, const uint8_t* extra, int H, int I, uint8_t* base, WmStamp* out) {
+  static_assert(sizeof(CUtensorMap) == sizeof(ctx->wm_tpl[0].map), "hb_ctx::WmTemplate");
+  out->tab = tab; out->n_tab = n_tab; out->extra = extra;
+  out->dst[0] = base; out->dst[1] = base + wm_bytes(H);
+  out->nv[0] = wm_variants(H); out->nv[1] = wm_variants(I);
+  const int r = wm_template(ctx, H / 2, base, &out->tpl[0]);
+  return r ? r : wm_template(ctx, I / 2, base, &out->tpl[1]);
 }
 
-// the same maps for the prefill GEMM with bf16 activations, which streams raw code boxes through them
-int hbk_moe_dtc_maps(hb_ctx* ctx, const uint8_t* const* tab, int n_tab, const uint8_t* shared_rec, int H, int I, cudaStream_t st) {
-  return dtc_maps_for(ctx, tab, n_tab, shared_rec, H, I, st);
+// what both passes share: the list, the weight maps of the pass, the dividers
+static void dtc_args_common(hb_ctx* ctx, const DecodeWs& w, int kind, int K, const uint8_t* maps, int items_per_group, DtcArgs* a) {
+  a->hdr = w.hdr; a->groups = w.groups; a->down = kind; a->K = K; a->err = ctx->dev_err;
+  a->wm = wm_args(maps, K);
+  a->dIT.set((uint32_t)items_per_group); a->dG.set((uint32_t)dtc_grid(ctx));
 }
-void hbk_moe_dtc_map_set(const hb_ctx* ctx, int kind, const void** maps, const unsigned long long** anchor) {
-  const CUtensorMap* m = reinterpret_cast<const CUtensorMap*>(static_cast<const char*>(ctx->dtc_maps) + kind * kMapSetBytes);
-  *maps = m;
-  *anchor = &reinterpret_cast<const DtcMeta*>(m + DT_VMAX)->anchor;
-}
-int hbk_moe_dtc_vmax() { return DT_VMAX; }
 
 #ifdef HB_DTC_TRACE
 extern "C" __attribute__((visibility("default"))) int hb_dtc_trace_read(long long* out, int n) {
@@ -657,12 +597,13 @@ int hbk_moe_dtc_gu_run(hb_ctx* ctx, const void* x, int x_ld, int M, const uint8_
   dtc_carve(ws, hbk_moe_decode_ws_bytes(P, H, I) - hbk_moe_dtc_ws_extra(P, H, I), P, H, I, &dw);
   hb_rec_layout L;
   hb_rec_layout_make(H, I, &L);
-  int r = dtc_maps_for(ctx, tab, n_tab, shared_rec, H, I, st);
+  WmStamp wm;
+  int r = hbk_wm_stamp_args(ctx, tab, n_tab, shared_rec, H, I, dw.maps, &wm);
   if (r) return r;
-  XdigArgs xa{reinterpret_cast<const __nv_bfloat16*>(x), x_ld, H, dw.x, wait_flags, wait_n, wait_step, ctx->dev_err, 0};
-  if ((r = hb_launch(ctx, "moe_xdig", true, moe_xdig_kernel, dim3(M), dim3(256), 0, st, xa))) return r;
+  XdigArgs xa{reinterpret_cast<const __nv_bfloat16*>(x), x_ld, H, M, dw.x, wait_flags, wait_n, wait_step, ctx->dev_err, 0};
+  if ((r = hb_launch(ctx, "moe_xdig", true, moe_xdig_kernel, dim3(M + 1), dim3(256), 0, st, xa, wm))) return r;
   DtcArgs a{};
-  dtc_args_common(ctx, w, 0, H, I / DT_GU_ROWS, &a);
+  dtc_args_common(ctx, w, 0, H, dw.maps, I / DT_GU_ROWS, &a);
   a.s_row = w.s_row; a.out_ld = I; a.limit = limit;
   a.off_w = (uint32_t)L.w1; a.off_s0 = (uint32_t)L.s1; a.off_s1 = (uint32_t)L.s3; a.off_g = (uint32_t)L.g;
   a.row2 = (int)((L.w3 - L.w1) / (size_t)(H / 2)); a.trows = DT_GU_ROWS;
@@ -679,12 +620,11 @@ int hbk_moe_dtc_down_run(hb_ctx* ctx, int P, int H, int I, void* ws, const Reduc
   dtc_carve(ws, hbk_moe_decode_ws_bytes(P, H, I) - hbk_moe_dtc_ws_extra(P, H, I), P, H, I, &dw);
   hb_rec_layout L;
   hb_rec_layout_make(H, I, &L);
-  HB_REQUIRE(ctx, ctx->dtc_H == H && ctx->dtc_I == I, HB_ERR_INVALID, "moe_decode: the down pass on the tensor cores follows the gate/up pass of the same shape");
-  XdigArgs xa{w.y, I, I, dw.y, nullptr, 0, nullptr, ctx->dev_err, 1};
-  int r = hb_launch(ctx, "moe_ydig", true, moe_xdig_kernel, dim3(P), dim3(256), 0, st, xa);
+  XdigArgs xa{w.y, I, I, P, dw.y, nullptr, 0, nullptr, ctx->dev_err, 1};       // the gate/up pass of the same call has stamped the maps of both
+  int r = hb_launch(ctx, "moe_ydig", true, moe_xdig_kernel, dim3(P), dim3(256), 0, st, xa, WmStamp{});
   if (r) return r;
   DtcArgs a{};
-  dtc_args_common(ctx, w, 1, I, H / 128, &a);
+  dtc_args_common(ctx, w, 1, I, dw.maps + wm_bytes(H), H / 128, &a);
   a.s_row = nullptr; a.out_ld = H; a.limit = 0.f;
   a.off_w = (uint32_t)L.w2; a.off_s0 = (uint32_t)L.s2; a.off_s1 = (uint32_t)(L.s2 + (size_t)64 * (I / 16)); a.off_g = (uint32_t)L.g;
   a.row2 = 64; a.trows = 128;

@@ -569,6 +569,7 @@ namespace {
 struct PfWs {
   int* hist; int* n_slots; int* n_tiles; TileRef* tiles; int* perm; int* pos_of; CUtensorMap* tmB; __nv_bfloat16* y; __nv_bfloat16* part;
   uint8_t *yq, *ys, *xq_s, *xs_s; float *yg, *xg_s;
+  uint8_t* wmaps;
 };
 size_t pf_carve(void* ws, int S, int K, int E, int H, int I, PfWs* w) {
   size_t off = 0;
@@ -581,6 +582,7 @@ size_t pf_carve(void* ws, int S, int K, int E, int H, int I, PfWs* w) {
   t.y = (__nv_bfloat16*)take(P * I * 2); t.part = (__nv_bfloat16*)take(P * H * 2);
   t.xq_s = (uint8_t*)take(P * H / 2); t.xs_s = (uint8_t*)take(P * H / 16); t.xg_s = (float*)take(P * 4);
   t.yq = (uint8_t*)take(P * I / 2); t.ys = (uint8_t*)take(P * I / 16); t.yg = (float*)take(P * 4);
+  t.wmaps = (uint8_t*)take(wm_bytes(H) + wm_bytes(I));
   if (w) *w = t;
   return off;
 }
@@ -630,7 +632,8 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
   hb_rec_layout L;
   hb_rec_layout_make(H, I, &L);
   const int Kr = shared_pair ? K - 1 : K;                      // routed pairs of a row: what w holds
-  int r = hbk_moe_dtc_maps(ctx, lt, E, nullptr, H, I, st);
+  WmStamp wm;
+  int r = hbk_wm_stamp_args(ctx, lt, E, nullptr, H, I, W.wmaps, &wm);
   if (r) return r;
   const size_t Pcap = (size_t)S * K;
   CUtensorMap tm_x, tm_y;
@@ -638,16 +641,9 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
   if ((r = a16_make_map(ctx, &tm_y, W.y, (size_t)I, Pcap))) return r;
   const int grid = ctx->max_ctas > 0 && ctx->max_ctas < ctx->sm_count ? ctx->max_ctas : ctx->sm_count;
   auto common = [&](int kind, A16Args* a) {
-    const void* maps; const unsigned long long* anchor;
-    hbk_moe_dtc_map_set(ctx, kind, &maps, &anchor);
     const int Kd = kind ? I : H;
     a->tiles = W.tiles; a->n_tiles = W.n_tiles; a->perm = W.perm; a->tab = lt; a->down = kind; a->K = Kd; a->n_out = kind ? H : I;
-    a->maps = reinterpret_cast<const CUtensorMap*>(maps); a->anchor = anchor; a->vmax = hbk_moe_dtc_vmax();
-    a->pitch = Kd / 2;
-    int g = a->pitch, b = 4096;
-    while (b) { const int t2 = g % b; g = b; b = t2; }
-    a->gstep = g; a->pshift = -1;
-    for (int sft = 7; sft <= 12; ++sft) if (a->pitch == (1 << sft)) a->pshift = sft;
+    a->wm = wm_args(kind ? W.wmaps + wm_bytes(H) : W.wmaps, Kd);
     a->off_g = (uint32_t)L.g; a->limit = limit; a->err = ctx->dev_err;
   };
   for (int s0 = 0; s0 < M; s0 += S) {
@@ -663,8 +659,8 @@ int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids,
     if (plan_ctas > PLAN_MAX_CTAS) plan_ctas = PLAN_MAX_CTAS;
     if (plan_ctas > ctx->sm_count) plan_ctas = ctx->sm_count;
     if ((r = hb_launch(ctx, "pf_plan", false, pf_plan_kernel, dim3(plan_ctas), dim3(PLAN_THREADS), 0, st, pl))) return r;
-    if ((r = hb_launch(ctx, "a16_gather", false, a16_gather_kernel, dim3(P < ctx->sm_count * 16 ? P : ctx->sm_count * 16), dim3(256), 0, st, x + (size_t)s0 * H,
-                       (const int*)W.perm, (const int*)W.n_slots, K, H, W.part)))
+    if ((r = hb_launch(ctx, "a16_gather", false, a16_gather_kernel, dim3((P < ctx->sm_count * 16 ? P : ctx->sm_count * 16) + 1), dim3(256), 0, st, x + (size_t)s0 * H,
+                       (const int*)W.perm, (const int*)W.n_slots, K, H, W.part, wm)))
       return r;
     A16Args a{};
     common(0, &a);

@@ -14,14 +14,14 @@
 // shared memory (with one A tile per item the activation stream alone ran into what the SMs can pull out of L2).
 //
 // Per CTA (persistent, one per SM, 27 warps): warp 9 (one thread) streams by TMA the raw code boxes of the weights (128 bytes × 64
-// rows, 256 k values per row, through the anchored tensor map of the decode path), warp 26 the activation boxes (64 values × 64 rows of
+// rows, 256 k values per row, through the call's own weight maps, wmap.cuh), warp 26 the activation boxes (64 values × 64 rows of
 // bf16) of the tile; warps 10-25 (eight per A tile) turn a raw box into four operand tiles, fetching their row's block scales from
 // global memory a raw box ahead; warp 8 and warp 27 (one thread each) issue the MMAs of an A tile (128 × N × 16, four a step); warps 0-3 and 4-7 run
 // the epilogues of the two accumulators.  Gate/up: an A tile holds 64 gate and 64 up rows arranged so that lanes l and l + 16 of a
 // warp hold the gate and the up value of the same row of I — SwiGLU needs one exchange.  Every wait is bounded; a barrier gets one
 // arrival per warp, not per thread (arrivals on one barrier are taken one after the other).
 #pragma once
-#include "tc_common.cuh"
+#include "wmap.cuh"
 
 namespace hb {
 
@@ -65,8 +65,7 @@ struct A16Args {
   uint32_t off_w, off_s0, off_s1, off_g;        // record offsets: first matrix, scales of the matrix of lanes 0-15 / 16-31 of a warp (gate / up; down:
                                                 // the same matrix twice), global scales
   int row2;                                     // matrix rows between the two 64-row boxes of an A tile
-  const CUtensorMap* maps; const unsigned long long* anchor; int vmax;   // anchored weight map (variants) of this pass
-  int pitch, gstep, pshift;
+  WmArgs wm;                                    // the weight maps of this pass
   float limit;
   __nv_bfloat16* out;
   uint32_t* err;
@@ -123,11 +122,13 @@ __device__ __forceinline__ uint4 a16_dequant8(uint32_t w, uint32_t sv) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// The slot-ordered copy of the activation rows: row `slot` = x[perm[slot] / K].  One CTA per slot at a time.
+// The slot-ordered copy of the activation rows: row `slot` = x[perm[slot] / K].  One CTA per slot at a time; the last CTA stamps the weight
+// maps of both GEMMs instead.
 __global__ void __launch_bounds__(256) a16_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ perm, const int* __restrict__ n_slots, int K,
-                                                         int H, __nv_bfloat16* __restrict__ out) {
+                                                         int H, __nv_bfloat16* __restrict__ out, const __grid_constant__ WmStamp wm) {
+  if (blockIdx.x == gridDim.x - 1) { wm_stamp(wm); return; }
   const int n = *n_slots;
-  for (int s = blockIdx.x; s < n; s += gridDim.x) {
+  for (int s = blockIdx.x; s < n; s += gridDim.x - 1) {
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(perm[s] / K) * H);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)s * H);
     for (int i = threadIdx.x; i < H / 8; i += 256) dst[i] = __ldg(src + i);
@@ -185,29 +186,18 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
   if (warp == A16_W_TMA) {
     // ------------------------------------------------------------------------------------------------ raw code boxes: one thread
     if (elect_one()) {
-      uint32_t rit = 0, seen = 0u;
+      uint32_t rit = 0;
       bool ok = true;
       [[maybe_unused]] long long tw = 0, t0 = clock64();
-      const unsigned long long anchor = *a.anchor;
+      WmReader wm;
+      wm.init(a.wm);
       for (int item = blockIdx.x; item < n_items_all && ok; item += gridDim.x) {
         const int ti = item / nT, t = item - ti * nT;
         const TileRef tl = a.tiles[ti];
         const uint8_t* rec = a.tab[tl.expert];
-        const unsigned long long addr = reinterpret_cast<unsigned long long>(rec) + a.off_w, delta = addr - anchor;
-        unsigned long long row;
-        int v = 0;
-        if (!rec || addr < anchor) { atomicOr(a.err, 0x400000u); break; }
-        if (a.pshift >= 0) row = delta >> a.pshift;
-        else {
-          const unsigned long long rem = delta % (unsigned long long)a.pitch;
-          row = (delta - rem) / (unsigned long long)a.pitch;
-          v = (int)(rem / (unsigned long long)a.gstep);
-          if (rem % (unsigned long long)a.gstep || v >= a.vmax) { atomicOr(a.err, 0x400000u); break; }
-        }
-        if (row + (1ull << 24) >= (1ull << 31)) { atomicOr(a.err, 0x400000u); break; }
-        const CUtensorMap* map = a.maps + v;
-        if (!((seen >> v) & 1u)) { tmap_acquire(map); seen |= 1u << v; }
-        const int r0 = (int)row + 2 * t * arows;
+        WmBox box;
+        if (!rec || !wm.locate(rec + a.off_w, box, a.err)) break;
+        const int r0 = 2 * t * arows;
         for (int rs = 0; rs < nk / 4 && ok; ++rs, ++rit) {
           const uint32_t sl = rit % C::RAWS;
           A16_TIMED(tw, ok = mbar_wait(&emptyR[sl], ((rit / C::RAWS) & 1u) ^ 1u, a.err, 0x1u));
@@ -216,8 +206,8 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
           mbar_expect_tx(&fullR[sl], C::RAW);
 #pragma unroll
           for (int uu = 0; uu < 2; ++uu) {
-            tma_load_2d(rb + uu * C::A1, map, rs * 128, r0 + uu * arows, &fullR[sl]);
-            tma_load_2d(rb + uu * C::A1 + C::A1 / 2, map, rs * 128, r0 + uu * arows + a.row2, &fullR[sl]);
+            wm.load(rb + uu * C::A1, box, rs * 128, r0 + uu * arows, &fullR[sl]);
+            wm.load(rb + uu * C::A1 + C::A1 / 2, box, rs * 128, r0 + uu * arows + a.row2, &fullR[sl]);
           }
         }
       }
