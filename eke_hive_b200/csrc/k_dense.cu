@@ -87,7 +87,7 @@ struct DenseArgs {
   DenseMat mat[2]; int n_mats;
   uint32_t* err;                          // the context's error word (bounded waits)
   int N, K, M, ldx; uint32_t m_inv;        // m_inv: ceil(2^32 / M) for i / M (M > 1)
-  int sl0, slices;                        //         // this launch covers slices [sl0, sl0 + slices) of K / 256
+  int sl0, slices;                        // this launch covers slices [sl0, sl0 + slices) of K / 256
   const __nv_bfloat16* x;
   int mode; void* y; int ldy;             // 0: y fp32, 1: y bf16, 2: act = bf16( bf16(silu(bf16 gate)) · bf16 up )
   float4* acc; int acc_in, last;          // K beyond one launch: sums so far [strip][tile][lane], read if acc_in, written unless last
@@ -143,8 +143,8 @@ __device__ __forceinline__ void lb2_pairs(uint32_t w, uint32_t base, uint32_t (&
 }
 
 struct DenseSmem { size_t sums, inv, xch, bars, ring, total; };   // byte offsets; the fragments come first
-__host__ __device__ inline DenseSmem dense_smem(int fmt, int nb, int mt, int slices, int cluster, int nst) {
-  DenseSmem s;
+__host__ __device__ constexpr DenseSmem dense_smem(int fmt, int nb, int mt, int slices, int cluster, int nst) {
+  DenseSmem s{};
   size_t o = (size_t)slices * nb * mt * 512;
   s.sums = o; o += fmt == HB_FMT_NVFP4 ? 0 : (size_t)slices * nb * 256;
   s.inv = o; o += (size_t)slices * nb * 32;
@@ -508,6 +508,17 @@ int dense_cluster(const hb_ctx* ctx, int N, int n_mats, int slices) {
 constexpr int kLaunchSlices = kMaxSlices * kMaxCluster;    // slices one launch covers at most (K = 40960)
 int dense_launches(int K) { return (K / kDSlice + kLaunchSlices - 1) / kLaunchSlices; }
 
+// Eight rows fit beside the shallower ring whatever share of the columns dense_cluster gives a CTA, so every call has a way to run.  Two column
+// tiles do not: 20 slices of a 9-16 row call take 160 KB of fragments, and a cluster's exchange buffer leaves too little for three stages
+// (NVFP4 236928 and 3 bits 234880 of 232448 bytes).
+constexpr bool dense_eight_rows_fit() {
+  for (int fmt = 0; fmt < 3; ++fmt)
+    for (int c = 1; c <= kMaxCluster; c *= 2)
+      if (dense_smem(fmt, 1, 8, kMaxSlices, c, 3).total > 227 * 1024) return false;
+  return true;
+}
+static_assert(HB_FMT_NVFP4 < 3 && HB_FMT_LB3_G64 < 3 && HB_FMT_LB2_G64 < 3 && dense_eight_rows_fit(), "shared memory");
+
 using DenseFn = void (*)(const DenseArgs);
 struct DenseKernel { DenseFn fn; int nst; };
 // the ring depths built for a format, deepest first: 64-150 KB of weights in flight on an SM
@@ -523,6 +534,13 @@ void dense_kernels(int fmt, int nb, DenseKernel (&k)[2]) {
   else dense_kernels<HB_FMT_LB3_G64>(nb, k);
 }
 
+// the deepest of the built rings that fits with M rows and `per` slices a CTA, -1: none
+int dense_depth(const hb_ctx* ctx, int fmt, int M, int per, int C, const DenseKernel (&k)[2], size_t* smem) {
+  for (int v = 0; v < 2; ++v)
+    if ((*smem = dense_smem(fmt, M > 8 ? 2 : 1, M < 8 ? M : 8, per, C, k[v].nst).total) <= (size_t)ctx->smem_optin) return v;
+  return -1;
+}
+
 int dense_run(hb_ctx* ctx, const hb_qmat* A, const hb_qmat* B2, const void* x, int ldx, int M, int mode, void* y, int ldy, void* ws, cudaStream_t st) {
   const int fmt = A->fmt, slices = A->K / kDSlice, nb = M > 8 ? 2 : 1, launches = dense_launches(A->K);
   DenseArgs a{};
@@ -532,13 +550,24 @@ int dense_run(hb_ctx* ctx, const hb_qmat* A, const hb_qmat* B2, const void* x, i
   a.mode = mode; a.y = y; a.ldy = ldy; a.err = ctx->dev_err;
   DenseKernel k[2];
   dense_kernels(fmt, nb, k);
+  auto split = [&](int i, int* sl0, int* n) { *sl0 = (int)((long long)slices * i / launches); *n = (int)((long long)slices * (i + 1) / launches) - *sl0; };
+  for (int i = 0; i < launches; ++i) {                                       // before anything runs: does every launch fit?
+    int sl0, n; size_t smem;
+    split(i, &sl0, &n);
+    const int C = dense_cluster(ctx, A->N, a.n_mats, n);
+    if (dense_depth(ctx, fmt, M, (n + C - 1) / C, C, k, &smem) >= 0) continue;
+    HB_REQUIRE(ctx, M > 8, HB_ERR_UNSUPPORTED, "dense_gemv: N=%d K=%d needs %zu bytes of shared memory", A->N, A->K, smem);
+    // two column tiles do not fit: the first eight rows and the rest one after the other.  The split of the columns stays the matrix's, so
+    // the sums are the same.
+    const int r = dense_run(ctx, A, B2, x, ldx, 8, mode, y, ldy, ws, st);
+    return r ? r : dense_run(ctx, A, B2, a.x + 8 * (size_t)ldx, ldx, M - 8, mode, static_cast<char*>(y) + 8 * (size_t)ldy * (mode == 0 ? 4 : 2), ldy, ws, st);
+  }
   for (int i = 0; i < launches; ++i) {
-    a.sl0 = (int)((long long)slices * i / launches); a.slices = (int)((long long)slices * (i + 1) / launches) - a.sl0;
+    split(i, &a.sl0, &a.slices);
     a.acc = launches > 1 ? reinterpret_cast<float4*>(ws) : nullptr; a.acc_in = i > 0; a.last = i == launches - 1;
     const int C = dense_cluster(ctx, A->N, a.n_mats, a.slices), per = (a.slices + C - 1) / C;
-    int v = 0;
-    size_t smem = dense_smem(fmt, nb, M < 8 ? M : 8, per, C, k[0].nst).total;
-    if (smem > (size_t)ctx->smem_optin) { v = 1; smem = dense_smem(fmt, nb, M < 8 ? M : 8, per, C, k[1].nst).total; }
+    size_t smem;
+    const int v = dense_depth(ctx, fmt, M, per, C, k, &smem);
     const int strips = B2 ? (A->N + 7) / 8 : (A->N + 15) / 16, most = ctx->dense_clusters[C == 1 ? 0 : C == 2 ? 1 : C == 4 ? 2 : 3];
     const int ncl = most < strips ? most : strips;
     const int r = hb_launch_cluster(ctx, fmt == HB_FMT_NVFP4 ? "dense_gemv_nvfp4" : fmt == HB_FMT_LB2_G64 ? "dense_gemv_lb2" : "dense_gemv_lb3", true, C, k[v].fn,

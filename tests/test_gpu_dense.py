@@ -151,3 +151,47 @@ def test_dense_gemv_splits_and_tiles(E, oracle, fmt, N, K, M):
     rmsa = np.sqrt(np.mean(refa.astype(np.float64) ** 2))
     assert np.all(np.abs(act - refa) <= 2.0 ** -7 * (amp + 3.0) * np.abs(refa) + 5e-3 * rmsa)
     E.context().check_device()
+
+
+@pytest.mark.parametrize("fmt", ["nvfp4", "lb3", "lb2"])
+@pytest.mark.parametrize("N,K", [(8192, 10240), (4096, 20480), (40, 39168), (24, 40960), (8, 79872), (9, 81920)])
+def test_dense_gemv_longest_column_share(E, oracle, fmt, N, K):
+    """K that gives a CTA the most columns its shared memory takes (20 slices of 256), with 2, 4 and 8 CTAs sharing K and over two launches, at 8, 9
+    and 16 rows: two column tiles' fragments do not always fit beside the exchange buffer there.  A row's bits are those of the row alone, sampled
+    matrix rows are compared with the oracle (bound as in test_dense_gemv_splits_and_tiles)."""
+    import torch
+    rng = np.random.default_rng(N + K)
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    pick = np.unique(np.concatenate([[0, N - 1], rng.integers(0, N, 14)]))
+    at = torch.from_numpy(pick).cuda()
+
+    def matrix():
+        if fmt == "nvfp4":
+            q = torch.randint(0, 256, (N, K // 2), generator=g, device="cuda", dtype=torch.uint8)
+            s = torch.randint(0x28, 0x48, (N, K // 16), generator=g, device="cuda", dtype=torch.uint8)
+            ref = lambda x: oracle.gemv_nvfp4(q[at].cpu().numpy(), s[at].cpu().numpy(), 0.003, x)
+            return E.GMat(E.FMT_NVFP4, N, K, q, s, None, 0.003), ref
+        bits = 3 if fmt == "lb3" else 2
+        q = torch.randint(0, 256, (N * K * bits // 8,), generator=g, device="cuda", dtype=torch.uint8)
+        s = (torch.rand((N, K // 64), generator=g, device="cuda") * 0.02 + 0.01).half()
+        zp = (torch.rand((N, K // 64), generator=g, device="cuda") * (2 ** bits - 1)).half()
+        sub = q[:N * K // 4].reshape(N, -1)[at].reshape(-1)
+        if bits == 3:
+            sub = torch.cat((sub, q[N * K // 4:].reshape(N, -1)[at].reshape(-1)))
+        host = [t.contiguous().cpu().numpy() for t in (sub, s[at].view(torch.int16), zp[at].view(torch.int16))]
+        ref = lambda x: oracle.lb_gemv(host[0], host[1].view(np.float16), host[2].view(np.float16), bits, x)
+        return E.GMat(E.FMT_LB3_G64 if bits == 3 else E.FMT_LB2_G64, N, K, q, s, zp), ref
+
+    (G, refg), (U, _) = matrix(), matrix()
+    x = oracle.bf16r(rng.normal(0, 1, (16, K)).astype(np.float32))
+    xd = bf16_tensor(x)
+    y8, a8 = [torch.cat([f(xd[:8]), f(xd[8:])]) for f in (lambda v: E.dense_gemv(G, v), lambda v: E.dense_gemv_gu(G, U, v))]
+    for M in (9, 16):
+        assert torch.equal(E.dense_gemv(G, xd[:M]), y8[:M])
+        yb = E.dense_gemv(G, xd[:M], out_dtype=torch.bfloat16)
+        assert torch.equal(yb.view(torch.int16), y8[:M].bfloat16().view(torch.int16))
+        assert torch.equal(E.dense_gemv_gu(G, U, xd[:M]).view(torch.int16), a8[:M].view(torch.int16))
+    E.context().check_device()
+    ref = refg(x[[0, 8, 15]])
+    rms = np.sqrt(np.mean(ref.astype(np.float64) ** 2))
+    assert np.max(np.abs(y8[[0, 8, 15]][:, at].cpu().numpy() - ref)) <= 2e-3 * rms
