@@ -131,7 +131,12 @@ __device__ __forceinline__ void group_body(const GroupArgs& a) {
     uint32_t kk = ~0u;
     if (!routed) {
       const uint8_t* r = recs[i];
-      if (r) { kk = (uint32_t)i; for (int j = 0; j < i; ++j) if (recs[j] == r) { kk = (uint32_t)j; break; } }   // the first pair with this record stands for it
+      if (r) {                                          // the first pair with this record stands for it; eight looked at together: one at a time is a load's latency each
+        kk = (uint32_t)i;
+        for (int j0 = 0; j0 < i && kk == (uint32_t)i; j0 += 8)
+#pragma unroll
+          for (int u = 7; u >= 0; --u) { const int j = min(j0 + u, i); if (recs[j] == r) kk = (uint32_t)j; }
+      }
     } else if (i < MK) kk = key[i] < (uint32_t)a.E ? key[i] + 1u : ~0u;
     else {                                              // one pair of weight 1 per row for the shared expert
       const int row = i - MK;

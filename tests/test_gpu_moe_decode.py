@@ -132,6 +132,27 @@ def test_pair_list_accumulates_in_pair_order(E, oracle):
     assert rel_rms_err(out.cpu().numpy(), ref) <= TOL
 
 
+@pytest.mark.parametrize("n", [1, 8, 9, 17, 513, 2048, 4096])
+def test_long_pair_lists_equal_their_pieces(E, oracle, n):
+    """A list in one call and the same list in calls of 64 pairs add up the same numbers in the same order, so they agree bit for bit: the grouping
+    finds the first pair of every record however far back it is."""
+    import torch
+    H, I = 256, 256
+    drecs = upload(random_records(oracle, H, I, 40, seed=3))
+    rng = np.random.default_rng(n)
+    x = bf16_tensor(oracle.bf16r(rng.normal(0, 1, (50, H)).astype(np.float32)))
+    which = rng.integers(-1, 40, n)
+    which[-1] = which[0]
+    pairs = E.make_pairs(rng.integers(0, 50, n), [None if e < 0 else drecs[e] for e in which], rng.uniform(0.1, 0.9, n).astype(np.float32), "cuda")
+    one, many = (torch.zeros((50, H), dtype=torch.float32, device="cuda") for _ in range(2))
+    E.moe_decode(pairs, x, H, I, 0.0, one)
+    for a in range(0, n, 64):
+        E.moe_decode(pairs[a:a + 64], x, H, I, 0.0, many)
+    torch.cuda.synchronize()
+    E.context().check_device()
+    assert torch.equal(one, many)
+
+
 def test_outlier_activations_stay_finite(E, oracle):
     """Activations far outside the f16 range (±3e5, the reference's own case in engine/tests/test_glm_moe.cu): the streaming path
     rescales each row slice by a power of two, so results stay finite and within tolerance."""
