@@ -176,3 +176,28 @@ def test_quantize_bits_at_the_rounding_edges(E, oracle, N, K):
     q, s, g = E.nvfp4_quantize(torch.from_numpy(small).cuda())
     q0, s0, g0 = oracle.nvfp4_quantize(small, search=False)
     assert np.array_equal(s.cpu().numpy(), s0) and np.float32(g.item()).tobytes() == np.float32(g0).tobytes()
+
+
+def test_quantize_signs_of_zero_and_overflowing_scale(E):
+    """What the two comparisons with the numpy rule leave out.  A value that rounds to zero keeps its sign in the code (8 for a negative one, -0
+    too), a block without a scale has codes 0.  Where the global scale overflows to infinity (largest magnitude below 2688 / 2^128), every block scale
+    saturates to 448; a value times infinity over 448 saturates to the largest code with the value's sign, and a zero times infinity is NaN, which
+    the converter turns into the largest positive code."""
+    import torch
+    w = torch.zeros((4, 64))
+    w[0, 0] = 2688.0 * 2.0 ** -7                                   # global scale 2^7
+    w[0, 16:32] = torch.tensor([6.0, -0.0, 0.0, -0.2, 0.2, -1e-30, 1e-30, -1e-45, 0.24, -0.24, 0.25, -0.25, -0.26, 0.26, -6.0, 1.0]) * 2.0 ** -7
+    w[1, 0:16] = -1e-7                                             # block scale rounds to zero
+    q, s, g = (t.cpu() for t in E.nvfp4_quantize(w.cuda()))
+    code = torch.stack((q & 15, q >> 4), -1).reshape(4, 64)
+    assert code[0, 16:32].tolist() == [7, 8, 0, 8, 0, 8, 0, 8, 0, 8, 0, 8, 9, 1, 15, 2]
+    assert s[1, 0] == 0 and code[1, :16].tolist() == [0] * 16 and code[2].tolist() == [0] * 64
+    tiny = torch.zeros((2, 32))
+    tiny[0, :16] = torch.tensor([1.0, -1.0, 0.5, -0.25, 1e-3, -1e-3, 0.0, -0.0] * 2) * 2.0 ** -130
+    tiny[1, 16] = -2.0 ** -131
+    q, s, g = (t.cpu() for t in E.nvfp4_quantize(tiny.cuda()))
+    code = torch.stack((q & 15, q >> 4), -1).reshape(2, 32)
+    assert s.tolist() == [[0x7E, 0x7F], [0x7F, 0x7E]]
+    assert code[0, :16].tolist() == [7, 15, 7, 15, 7, 15, 7, 7] * 2
+    assert code[1, 16:].tolist() == [15] + [7] * 15
+    assert float(g) > 0.0

@@ -74,7 +74,7 @@ def test_zipf_biased_routing_matches(E, oracle):
 
 @pytest.mark.parametrize("Ex", [16, 31, 255, 256, 257, 511, 512, 513, 1023, 1024])
 def test_router_register_widths(E, oracle, Ex):
-    """Every register width of the row routers at its edges (8, 16, 32 scores a lane), with whole groups of equal scores: ids and
+    """The stand-alone routers (one warp a row) at the edges of a lane's share of the experts, with whole groups of equal scores: ids and
     weights are integers and fp32 results of the same operations in the same order, so they are compared bit for bit."""
     import torch
     rng = np.random.default_rng(Ex)
@@ -92,3 +92,39 @@ def test_router_register_widths(E, oracle, Ex):
         ids, w = E.router_topk(torch.from_numpy(lg).cuda(), None if b is None else torch.from_numpy(b).cuda(), k, 2.5)
         i0, w0 = oracle.router_sigmoid_topk(lg, b, k, 2.5, 0)
         assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+
+
+@pytest.mark.parametrize("kind", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("Ex", [16, 31, 512, 1024])
+def test_layer_routing_at_every_group_width(E, oracle, kind, Ex):
+    """The routing inside the decode layer's grouping kernel: one CTA with 16 and 8 warps a row (1 and 2 rows), a cluster with 16, 8, 4 and 2 warps a
+    row (3-8, 9-16, 17-32, 33-64 rows; the last of each range leaves groups without a row).  Rows of equal scores and rows with one score above
+    all others have more than 64 candidates wherever there are that many experts.  Ids and weights bit for bit against the oracle."""
+    import torch
+
+    from util import bf16_tensor, random_records, upload
+    H, I, k = 256, 256, 16
+    keep = upload(random_records(oracle, H, I, 4, Ex))
+    tab = E.rec_table([keep[e % 3] for e in range(Ex)])
+    for M in (1, 2, 3, 8, 9, 16, 17, 32, 33, 45, 64):
+        rng = np.random.default_rng(1000 * M + Ex)
+        lg = rng.normal(0, 1, (M, Ex)).astype(np.float32)
+        lg[::2] = np.round(lg[::2] * 4) / 4                       # runs of equal scores
+        special = M - 1 if M < 9 else M - 2
+        lg[special] = 0.25                                        # all equal: the first k ids
+        if M > 2:
+            lg[1] = -np.inf if kind == "softmax" else -3.0
+            lg[1, Ex // 2] = 1.0                                  # one far above the others, which are equal
+        x = bf16_tensor(oracle.bf16r(rng.normal(0, 1, (M, H)).astype(np.float32)))
+        for variant in (0, 1):
+            if kind == "softmax":
+                ids, w, _ = E.moe_layer_decode(torch.from_numpy(lg).cuda(), x, tab, 0, Ex, k, H, I, shared_rec=keep[3], renorm=variant == 0, logits_bf16=variant == 0)
+                i0, w0 = oracle.router_softmax_topk(lg, k, variant == 0, variant == 0, 0)
+            else:
+                bias = None if variant else (np.round(rng.normal(0, 1, Ex) * 2) / 2).astype(np.float32)
+                ids, w, _ = E.moe_layer_decode(torch.from_numpy(lg).cuda(), x, tab, 0, Ex, k, H, I, shared_rec=keep[3],
+                                               bias=None if bias is None else torch.from_numpy(bias).cuda(), sigmoid_scale=2.5)
+                i0, w0 = oracle.router_sigmoid_topk(lg, bias, k, 2.5, 0)
+            assert np.array_equal(ids.cpu().numpy(), i0), (M, variant)
+            assert w.cpu().numpy().tobytes() == w0.tobytes(), (M, variant)
+    E.context().check_device()
