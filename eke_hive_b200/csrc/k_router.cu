@@ -18,7 +18,8 @@ __global__ void router_kernel(const RouteArgs a, const float* __restrict__ logit
   const int m = blockIdx.x * kRouterWarps + warp;
   if (m >= M) return;
   int id; float wv;
-  route_row<SIG>(a, logits + (size_t)m * ld, sm_p + (size_t)warp * a.E, rs[warp], RouteGroup{0, 1, 0}, lane, id, wv);
+  if (a.E <= 32) route_row32<SIG>(a, logits + (size_t)m * ld, lane, id, wv);
+  else route_row<SIG>(a, logits + (size_t)m * ld, sm_p + (size_t)warp * a.E, rs[warp], RouteGroup{0, 1, 0}, lane, id, wv);
   if (lane < a.k) { ids[(size_t)m * a.k + lane] = id; w[(size_t)m * a.k + lane] = wv; }
 }
 

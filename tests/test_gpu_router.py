@@ -128,3 +128,26 @@ def test_layer_routing_at_every_group_width(E, oracle, kind, Ex):
             assert np.array_equal(ids.cpu().numpy(), i0), (M, variant)
             assert w.cpu().numpy().tobytes() == w0.tobytes(), (M, variant)
     E.context().check_device()
+
+
+@pytest.mark.parametrize("Ex,k", [(1, 1), (2, 1), (7, 7), (8, 3), (32, 1), (32, 16), (33, 16)])
+def test_routers_of_few_experts(E, oracle, Ex, k):
+    """Up to 32 experts a row sits in the lanes of a warp: equal scores, one finite score, every expert picked, logits rows longer than E; one
+    expert more takes the general way."""
+    import torch
+    rng = np.random.default_rng(100 * Ex + k)
+    lg = (np.round(rng.normal(0, 1, (11, Ex + 2)) * 4) / 4).astype(np.float32)
+    lg[1] = 0.25
+    lg[2] = -np.inf; lg[2, Ex // 2] = 1.0
+    lg[3] = rng.normal(0, 30, Ex + 2)                            # scores that underflow beside the largest
+    for renorm, lbf in ((True, True), (False, False)):
+        ids, w = E.router_softmax_topk(torch.from_numpy(lg).cuda(), k, renorm, lbf, E=Ex)
+        i0, w0 = oracle.router_softmax_topk(lg, k, renorm, lbf, 0, E=Ex)
+        assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+    ls = np.ascontiguousarray(lg[:, :Ex])
+    ls[2] = 0.5
+    bias = (np.round(rng.normal(0, 1, Ex) * 2) / 2).astype(np.float32)
+    for b in (bias, None):
+        ids, w = E.router_topk(torch.from_numpy(ls).cuda(), None if b is None else torch.from_numpy(b).cuda(), k, 2.5)
+        i0, w0 = oracle.router_sigmoid_topk(ls, b, k, 2.5, 0)
+        assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
