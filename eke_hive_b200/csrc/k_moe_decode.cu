@@ -33,12 +33,14 @@ struct GroupArgs {
   uint32_t k_inv;       // ceil(2^32 / K): i / K is the high word of i · k_inv (i, K ≤ HB_MAX_PAIRS; not for K = 1)
 };
 
-// Where the gate/up pass of an unpinned context runs on the tensor-memory kernel.  One GPU: from kTcGuMinWork = pairs · H · I on; below it the
-// kernel's start-up (tensor-memory allocation, work table, first boxes) costs what its faster stream saves.  Measured per layer, tensor
-// memory against register kernels: hidden 2048, intermediate 512, top-10 + shared: 1 row (11 pairs) 23.3 / 22.6 us, 2 rows 26.8 / 29.3,
-// 16 rows 64.6 / 76.4, 64 rows 137 / 169; hidden 4096, intermediate 1536, top-8 + shared: 1 row 36.4 / 38.0, 8 rows 45 / 52, 64 rows 150 / 196.
+// Where the gate/up pass of an unpinned context runs on the tensor-memory kernel.  One GPU: from kTcGuMinPairs pairs on, or from kTcGuMinWork =
+// pairs · H · I on; below both the kernel's start-up (tensor-memory allocation, work table, first boxes) costs what its faster stream saves.
+// Measured per layer, register kernels / tensor memory: hidden 2048, intermediate 512, top-10 + shared: 1 row (11 pairs) 22.6 / 23.0 us, 2 rows
+// 29.3 / 28.1, 16 rows 76.1 / 64.6, 64 rows 167 / 133; hidden 4096, intermediate 1536, top-8 + shared: 1 row 38.5 / 36.1, 8 rows 52 / 47, 64
+// rows 198 / 151.  Small matrices, where 40 pairs are less work than that: 512 x 512, 32 experts, 40 pairs 25.0 / 21.2; 512 x 256, 64 experts,
+// 126 pairs 27.3 / 22.3, 16 experts, 96 pairs 23.7 / 21.3; 256 x 256, 16 experts, 48 pairs 20.6 / 19.4, 64 experts, 72 pairs 19.7 / 19.7.
 constexpr long long kTcGuMinWork = 16ll << 20;
-constexpr int kTcGuMinPairs = 40;                   // expert parallel: this rank's share of the pairs
+constexpr int kTcGuMinPairs = 40;                   // under expert parallelism: this rank's share of the pairs, and up to 64 gathered rows
 
 // Sorts the pairs by expert: counts the pairs of every expert, scans the counts, places the pairs.  It sits alone on the critical path in
 // front of the two weight passes, so what bounds it is its chain of loads, instructions and block barriers: the counters are cleared
@@ -618,16 +620,16 @@ int hbk_moe_decode_run(hb_ctx* ctx, const hbk_pair_src& src, const void* x, int 
   ga.ld_ids = src.ld_ids ? src.ld_ids : src.K; ga.sh_row0 = src.sh_row0; ga.sh_rows = src.sh_rows < 0 ? src.M : src.sh_rows;
   ga.wait_flags = src.wait_flags; ga.wait_n = src.wait_n; ga.wait_step = src.wait_step; ga.wait_err = ctx->dev_err;
   // Which gate/up engine: a context may pin either (HB_FLAG_DECODE_MMA_SYNC / HB_FLAG_DECODE_TC_GU); unpinned, the size of the call decides
-  // (kTcGuMinWork).  Expert parallel (rows of all ranks, most pairs dead on this rank): what counts is this rank's share of the pairs, and
-  // with many gathered rows the digit planes of rows this rank has nothing for cost more than the faster stream saves (measured at 8
-  // ranks × 16 rows: 109 vs 99 µs per layer; at 4 ranks × 16 rows: 99 vs 103 µs; at 2 ranks: 101 vs 108 µs) — unpinned contexts take the
-  // tensor-memory kernel up to 64 gathered rows.
+  // (see kTcGuMinWork).  Expert parallel (rows of all ranks, most pairs dead on this rank): what counts is this rank's share of the pairs, and
+  // with many gathered rows the digit planes of rows this rank has nothing for cost more than the faster stream saves — unpinned contexts take
+  // the tensor-memory kernel up to 64 gathered rows.  (That line was measured with this kernel's first form, groups of two rows: 8 ranks × 16
+  // rows 109 vs 99 µs per layer, 4 ranks 99 vs 103, 2 ranks 101 vs 108.  It has not been measured since.)
   bool tc_gu = false;
   if (routed && !src.ws_stream_only && src.tab && hbk_moe_decode_fast(H, I) && hbk_moe_dtc_supported(H, I) && hbk_moe_dtc_gu_fits(ctx, P, src.E, H, I) &&
       !(ctx->flags & (HB_FLAG_DECODE_MMA_SYNC | HB_FLAG_FUSED))) {
     const int ranks = red.ep ? red.ep->world : 1;
     const int pairs = P > src.pairs_hint ? P : src.pairs_hint;
-    const bool auto_tc = ranks == 1 ? (long long)pairs * H * I >= kTcGuMinWork : pairs / ranks >= kTcGuMinPairs && src.M <= 64;
+    const bool auto_tc = ranks == 1 ? pairs >= kTcGuMinPairs || (long long)pairs * H * I >= kTcGuMinWork : pairs / ranks >= kTcGuMinPairs && src.M <= 64;
     tc_gu = (ctx->flags & (HB_FLAG_DECODE_TC_GU | HB_FLAG_DECODE_TC)) || auto_tc;
   }
   const int x_ld = src.x_ld ? src.x_ld : H;

@@ -51,7 +51,7 @@ typedef struct hb_config {
 #define HB_FLAG_DECODE_TC 16      /* same as HB_FLAG_DECODE_TC_GU (kept for callers that set it) */
 #define HB_FLAG_DECODE_TC_GU 64   /* decode, routed operators: the gate/up pass runs on the tensor-memory kernel (exact digit planes of the activations,
                                      block-scaled FP4 MMAs) at every size, grouping and down pass on the streaming kernels.  With neither flag the
-                                     library picks by the size of the call (pairs · H · I of 16 Mi or more: tensor memory); both engines meet the same
+                                     library picks by the size of the call (40 pairs, or pairs · H · I of 16 Mi, or more: tensor memory); both engines meet the same
                                      tolerance, and a row's bits do not depend on its batch as long as the engine does not change — pin one
                                      with a flag where that matters */
 #define HB_FLAG_DECODE_TC_DOWN 128 /* decode, routed operators on one GPU: where the gate/up pass runs on the tensor-memory kernel, the down pass does too

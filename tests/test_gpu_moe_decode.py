@@ -334,12 +334,13 @@ def test_glm_shaped_layer_with_zipf_bias(E, oracle, eng):
     eng.check_device()
 
 
-@pytest.mark.parametrize("M,K", [(5, 3), (4, 4), (1, 15), (1, 16)])
-def test_engine_of_an_unpinned_context(E, oracle, M, K):
-    """Either side of pairs · H · I = 16 Mi (2048 x 512: 16 pairs): an unpinned context gives the bits of the register kernels below it and of the
-    tensor-memory kernel from it on, and both stay inside the gate of the oracle."""
+@pytest.mark.parametrize("H,I,M,K", [(2048, 512, 5, 3), (2048, 512, 4, 4), (2048, 512, 1, 15), (2048, 512, 1, 16), (512, 256, 13, 3), (512, 256, 8, 5)])
+def test_engine_of_an_unpinned_context(E, oracle, H, I, M, K):
+    """Either side of pairs · H · I = 16 Mi (2048 x 512: 16 pairs) and of 40 pairs: an unpinned context gives the bits of the register kernels below
+    both and of the tensor-memory kernel from either on, and both kernels stay inside the gate of the oracle."""
     import torch
-    H, I, Ex = 2048, 512, 20
+    Ex = 20
+    on_tc = M * K * H * I >= 16 << 20 or M * K >= 40
     rng = np.random.default_rng(M * 100 + K)
     recs = random_records(oracle, H, I, Ex, seed=K)
     drecs = upload(recs)
@@ -349,7 +350,7 @@ def test_engine_of_an_unpinned_context(E, oracle, M, K):
     args = (torch.from_numpy(ids_np).cuda(), torch.from_numpy(w_np).cuda(), tab, 0, Ex, bf16_tensor(x_np), H, I)
     free, reg, tc = E.Context(), E.Context(flags=E.HB_FLAG_DECODE_MMA_SYNC), E.Context(flags=E.HB_FLAG_DECODE_TC_GU)
     outs = []
-    for c, name in ((free, "moe_gate_up_tc" if M * K * H * I >= 16 << 20 else "moe_gate_up"), (reg, "moe_gate_up"), (tc, "moe_gate_up_tc")):
+    for c, name in ((free, "moe_gate_up_tc" if on_tc else "moe_gate_up"), (reg, "moe_gate_up"), (tc, "moe_gate_up_tc")):
         outs.append(E.moe_decode_routed_f32(*args, ctx=c))
         c.profile(True)                                             # the same call once more, kernel by kernel
         assert torch.equal(E.moe_decode_routed_f32(*args, ctx=c), outs[-1])
@@ -357,6 +358,6 @@ def test_engine_of_an_unpinned_context(E, oracle, M, K):
         c.check_device()
         c.close()
     out, by_reg, by_tc = outs
-    assert torch.equal(out, by_tc if M * K * H * I >= 16 << 20 else by_reg)
+    assert torch.equal(out, by_tc if on_tc else by_reg)
     ref = oracle.moe_routed(H, I, ids_np, w_np, recs, x_np, 0.0, 0)
     assert max(rel_rms_err(by_reg.cpu().numpy(), ref), rel_rms_err(by_tc.cpu().numpy(), ref)) <= TOL
