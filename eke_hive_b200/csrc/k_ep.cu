@@ -223,6 +223,8 @@ int hb_ep_create(hb_ctx* ctx, int rank, int world, int B, int H, int K, void* co
   if (!ctx || !out) return HB_ERR_INVALID;
   HB_REQUIRE(ctx, world >= 1 && world <= kEpMaxRanks && rank >= 0 && rank < world && B >= 1 && H >= 8 && H % 8 == 0 && K >= 1 && recv && ag_flag && rs &&
                       rs_flag, HB_ERR_INVALID, "ep_create: rank %d of %d, B=%d H=%d K=%d", rank, world, B, H, K);
+  // 48 KB of dynamic shared memory beside the router's own arrays: what hb_ep_route_push accepts
+  HB_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(ep_route_push_kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024));
   hb_ep* e = new hb_ep();
   e->ctx = ctx; e->rank = rank; e->world = world; e->B = B; e->H = H; e->K = K; e->rec_bytes = (int)hb_ep_rec_bytes(H, K);
   for (int p = 0; p < world; ++p) {

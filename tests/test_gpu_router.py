@@ -151,3 +151,28 @@ def test_routers_of_few_experts(E, oracle, Ex, k):
         ids, w = E.router_topk(torch.from_numpy(ls).cuda(), None if b is None else torch.from_numpy(b).cuda(), k, 2.5)
         i0, w0 = oracle.router_sigmoid_topk(ls, b, k, 2.5, 0)
         assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+
+
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 5, 33, 700])
+def test_route_and_push_of_one_rank(E, oracle, B):
+    """The expert-parallel route + push kernel with a single rank (nothing to wait for): 16, 8, 4 and 2 warps a row, and the most rows its
+    shared memory takes (700 rows of 8 picks beside 16 experts' scores).  Rows, ids and weights arrive as the router gives them."""
+    import torch
+    H, Ex, k = 64, 16 if B == 700 else 160, 8
+    rng = np.random.default_rng(B)
+    lg = rng.normal(0, 1, (B, Ex)).astype(np.float32)
+    lg[-1] = 0.5
+    x = torch.from_numpy(rng.normal(0, 1, (B, H)).astype(np.float32)).bfloat16().cuda()
+    mine = torch.zeros(E.PeerExchange.layout(1, B, H, k)[1], dtype=torch.uint8, device="cuda")
+    ex = E.PeerExchange(mine, lambda o: [o], 0, 1, B, H, k)
+    ids, w = torch.zeros((B, k), dtype=torch.int32, device="cuda"), torch.zeros((B, k), device="cuda")
+    ex.route_push(torch.from_numpy(lg).cuda(), x, ids, w, Ex)
+    torch.cuda.synchronize()
+    i0, w0 = oracle.router_softmax_topk(lg, k, True, True, 0)
+    assert np.array_equal(ids.cpu().numpy(), i0) and w.cpu().numpy().tobytes() == w0.tobytes()
+    rec = mine[ex.off["recv"]:ex.off["recv"] + B * ex.rec_bytes].reshape(B, ex.rec_bytes)
+    assert torch.equal(rec[:, :2 * H].contiguous().view(torch.int16), x.view(torch.int16))
+    assert torch.equal(rec[:, 2 * H:2 * H + 4 * k].contiguous().view(torch.int32), ids)
+    assert torch.equal(rec[:, 2 * H + 4 * k:2 * H + 8 * k].contiguous().view(torch.float32), w)
+    E.context().check_device()
+    ex.close()
