@@ -521,7 +521,8 @@ static_assert(HB_FMT_NVFP4 < 3 && HB_FMT_LB3_G64 < 3 && HB_FMT_LB2_G64 < 3 && de
 
 using DenseFn = void (*)(const DenseArgs);
 struct DenseKernel { DenseFn fn; int nst; };
-// the ring depths built for a format, deepest first: 64-150 KB of weights in flight on an SM
+// The ring depths built for a format, deepest first.  An SM's rings hold, NVFP4 / 3 / 2 bits: one column tile (16 warps) 147 / 115 / 123 KB, shallow
+// 111 / 86 / 61; two (8 warps) 74 / 57 / 41 KB, shallow 55 / 43 / 31; all stages but one are in flight.
 template <int FMT>
 void dense_kernels(int nb, DenseKernel (&k)[2]) {
   constexpr int D = FMT == HB_FMT_LB2_G64 ? 6 : 4;

@@ -51,7 +51,7 @@ static_assert(PF_SF_COL0 + 48 * PF_ST <= PF_TMEM_COLS, "tensor memory");
 static_assert(PF_STAGE % 1024 == 0, "stage buffers must keep the 1024-byte alignment of the swizzle atom");
 static_assert(PF_SMEM <= 227 * 1024, "shared memory");
 
-struct TileRef { int slot0, rows, expert; };   // 128 consecutive slots (or fewer) of one expert's run of the sorted pairs (256 for the bf16-activation GEMM)
+struct TileRef { int slot0, rows, expert; };   // up to 128 consecutive slots of one expert's run of the sorted pairs (the bf16-activation GEMM: up to 64, 128 or 256)
 }  // namespace hb
 #include "pf_a16.cuh"
 namespace hb {
@@ -625,7 +625,7 @@ A16Kernel a16_kernel(int bn) {
                                                                                               : A16Kernel{a16_gemm_kernel<256>, (size_t)A16Cfg<256>::SMEM, 256};
 }
 
-// bf16 activations on the tensor cores: plan (tiles of ≤ 256 pairs) → slot-ordered copy of the rows → gate/up GEMM → down GEMM → sums.
+// bf16 activations on the tensor cores: plan (tiles of ≤ 64, 128 or 256 pairs) → slot-ordered copy of the rows → gate/up GEMM → down GEMM → sums.
 // The copy of the rows lives in the buffer of the per-pair down rows: the gate/up GEMM has read it before the down GEMM writes there.
 int pf_a16_run(hb_ctx* ctx, const uint8_t* const* lt, int E, const int32_t* ids, const float* w, int M, int K, const __nv_bfloat16* x, int H, int I, float limit,
                float* out, const PfWs& W, int S, cudaStream_t st, const hb_pf_combine* cmb, bool shared_pair = false) {

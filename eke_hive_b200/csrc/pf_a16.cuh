@@ -13,7 +13,7 @@
 // tensor memory and the MMAs of the next item wait for the epilogue.  Per 64 k values an item moves 32 KB of activations and 8 KB of codes from L2 into
 // shared memory (with one A tile per item the activation stream alone ran into what the SMs can pull out of L2).
 //
-// Per CTA (persistent, one per SM, 27 warps): warp 9 (one thread) streams by TMA the raw code boxes of the weights (128 bytes × 64
+// Per CTA (persistent, one per SM, 28 warps): warp 9 (one thread) streams by TMA the raw code boxes of the weights (128 bytes × 64
 // rows, 256 k values per row, through the call's own weight maps, wmap.cuh), warp 26 the activation boxes (64 values × 64 rows of
 // bf16) of the tile; warps 10-25 (eight per A tile) turn a raw box into four operand tiles, fetching their row's block scales from
 // global memory a raw box ahead; warp 8 and warp 27 (one thread each) issue the MMAs of an A tile (128 × N × 16, four a step); warps 0-3 and 4-7 run
@@ -51,7 +51,7 @@ struct A16Cfg {
   static constexpr int SMEM = 1024 + STA * A + STB * B + RAWS * RAW + 1024;
   static_assert(SMEM <= 227 * 1024 && ACOL + (AT ? STA * KA * 64 : 0) <= 512, "shared memory, tensor memory");
 };
-constexpr int A16_BN_MAX = 256, A16_BN_MIN = 64;
+constexpr int A16_BN_MIN = 64;
 constexpr int A16_THREADS = 28 * 32;            // warps 0-3 and 4-7 epilogues of the two A tiles, 8 and 27 their MMAs, 9 raw codes, 10-17 and 18-25 dequantisation, 26 activations
 constexpr int A16_W_MMA = 8, A16_W_TMA = 9, A16_W_DQ0 = 10, A16_W_ACT = 26, A16_W_MMA1 = 27, A16_DQ_THREADS = 512;
 constexpr int A16_TMEM_COLS = 512;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
   const uint32_t raw0 = smem_u32(a16_raw), base = (raw0 + 1023u) & ~1023u;
   uint8_t* sm = a16_raw + (base - raw0);
   uint8_t* smA = sm;                                   // [STA][2 A tiles][16 KB]
-  uint8_t* smB = smA + C::STA * C::A;                // [STB][32 KB]
+  uint8_t* smB = smA + C::STA * C::A;                // [STB][BN rows × 128 bytes]
   uint8_t* smR = smB + C::STB * C::B;                // [RAWS][2 A tiles][16 KB] raw codes
   uint64_t* fullA = reinterpret_cast<uint64_t*>(smR + C::RAWS * C::RAW);
   uint64_t* emptyA = fullA + C::STA;
@@ -434,8 +434,8 @@ __global__ void __launch_bounds__(A16_THREADS, 1) a16_gemm_kernel(const A16Args 
             float gv = hi ? got : v0, uv = hi ? v1 : got;
             if (a.limit > 0.f) { uv = fminf(fmaxf(uv, -a.limit), a.limit); gv = fminf(gv, a.limit); }
             // silu by the fast reciprocal (the decode kernels divide exactly; the difference is below the bf16 rounding that follows in
-            // all but a few cases in a thousand — the accumulators are not double-buffered, and the exact division's instructions
-            // were the longest part of the time the MMAs wait for this epilogue)
+            // all but a few cases in a thousand — with tiles of more than 64 pairs the accumulators are not double-buffered, and the exact
+            // division's instructions were the longest part of the time the MMAs wait for this epilogue)
             if (c0 + c + (hi ? 1 : 0) < tl.rows) orow[(size_t)c * a.n_out] = __float2bfloat16(__fdividef(gv, 1.f + __expf(-gv)) * uv);
           }
         }
