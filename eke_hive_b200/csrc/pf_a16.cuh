@@ -122,13 +122,13 @@ __device__ __forceinline__ uint4 a16_dequant8(uint32_t w, uint32_t sv) {
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// The slot-ordered copy of the activation rows: row `slot` = x[perm[slot] / K].  One CTA per slot at a time; the last CTA stamps the weight
-// maps of both GEMMs instead.
+// The slot-ordered copy of the activation rows: row `slot` = x[perm[slot] / K].  One CTA per slot at a time; the first CTA stamps the weight
+// maps of both GEMMs instead (the last one of a grid larger than the chip would start when the others are nearly done).
 __global__ void __launch_bounds__(256) a16_gather_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ perm, const int* __restrict__ n_slots, int K,
                                                          int H, __nv_bfloat16* __restrict__ out, const __grid_constant__ WmStamp wm) {
-  if (blockIdx.x == gridDim.x - 1) { wm_stamp(wm); return; }
+  if (blockIdx.x == 0) { wm_stamp(wm); return; }
   const int n = *n_slots;
-  for (int s = blockIdx.x; s < n; s += gridDim.x - 1) {
+  for (int s = blockIdx.x - 1; s < n; s += gridDim.x - 1) {
     const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(perm[s] / K) * H);
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)s * H);
     for (int i = threadIdx.x; i < H / 8; i += 256) dst[i] = __ldg(src + i);
